@@ -32,6 +32,7 @@
 #include "compact.cuh"
 
 #include "bulk.cuh"
+#include "lookback.cuh"
 
 #include <algorithm>
 
@@ -46,11 +47,6 @@ constexpr int CP_ITEMS_DIRECT = 8;
 constexpr int CP_ITEMS_STAGED = 4;
 // Largest staged tile (bytes of shared memory per CTA).
 constexpr uint32_t CP_STAGE_MAX = 48u << 10;
-constexpr ull LB_AGG = 1ull << 62;
-constexpr ull LB_INC = 2ull << 62;
-constexpr ull LB_VAL = (1ull << 62) - 1;
-constexpr uint32_t SPIN_LIMIT = 1u << 22;
-constexpr int LB_WINDOW = 8;  // look-back words read per round trip
 // Bulk-staged kernels: rows per thread by row width (bytes), and the largest
 // stage. Small tiles keep many CTAs (and their copies) in flight per SM.
 constexpr int CB_ITEMS_NARROW = 4;  // row_w <= 64: 1,024-row tiles (the vectorised count assumes 4)
@@ -58,6 +54,10 @@ constexpr int CB_ITEMS_WIDE = 2;    // row_w <= 128: 512-row tiles
 constexpr uint32_t CB_STAGE_MAX = 64u << 10;
 // Inputs from this many rows up take the two-pass form.
 constexpr uint64_t CB_TWO_PASS_ROWS = 1ull << 22;
+// The same for direct loads (a run-start list from a byte mask, say): its
+// tiles are short work, so the look-back bounds it (10M rows: one pass 94 us,
+// two 76 us).
+constexpr uint64_t CP_TWO_PASS_ROWS = 1ull << 20;
 
 struct CpArgs {
     CompactSpec sp;
@@ -66,8 +66,8 @@ struct CpArgs {
     uint32_t* status;
     uint32_t soff[CP_MAX_COLS];  // staged kernels: byte offset of each column's tile in shared memory
     uint32_t row_w;              // bytes per row over all columns
-    uint32_t* tile_cnt;          // two-pass form: kept rows per tile (pass 1)
-    ull* tile_off;               // two-pass form: output offset of each tile
+    uint32_t* tile_cnt;          // two-pass form: kept rows per tile (pass 1), then before it in its scan group
+    ull* group_tot;              // two-pass form: kept rows of each group of SCAN_TILES tiles
 };
 
 // Asynchronous global -> shared copy of one element (4, 8 or 16 bytes; both
@@ -165,56 +165,51 @@ __device__ __forceinline__ uint32_t cp_tile_scan(uint32_t (*cnt)[CP_NW]) {
     return local;
 }
 
-// Run by warp 0 after the tile's counts are in cnt: cp_tile_scan, then lane
-// 0 publishes the tile's count and looks back over the earlier tiles'
-// (status, value) words for the tile's output offset, left in *s_base.
+// Two-pass form: output offset of `tile` (and, in *total, of everything)
+// from the scanned counts: the totals of the earlier groups, added up by the
+// warp, and the offset within its group. Run by a whole warp.
+constexpr uint32_t SCAN_TILES = 4096;
+__device__ __forceinline__ ull cp_two_base(const CpArgs& a, uint32_t tile, uint32_t ntiles, ull* total) {
+    const uint32_t lane = lane_id(), g = tile / SCAN_TILES, ng = (ntiles + SCAN_TILES - 1) / SCAN_TILES;
+    ull before = 0, all = 0;
+    for (uint32_t i = lane; i < (total ? ng : g); i += 32) {
+        const ull v = a.group_tot[i];
+        all += v;
+        if (i < g) before += v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        before += __shfl_xor_sync(0xffffffffu, before, o);
+        if (total) all += __shfl_xor_sync(0xffffffffu, all, o);
+    }
+    if (total) *total = all;
+    return before + a.tile_cnt[tile];
+}
+
+// Scans the tile's counts in cnt, leaves its offset `base` (cp_two_base,
+// found while the tile's rows were on their way) in *s_base; the last tile
+// stores the total.
+template <int ITEMS>
+__device__ __forceinline__ void cp_two_offsets(const CpArgs& a, uint32_t tile, uint32_t ntiles, uint32_t (*cnt)[CP_NW],
+                                               ull base, ull* s_base) {
+    const uint32_t local = cp_tile_scan<ITEMS>(cnt);
+    if (lane_id() != 0) return;
+    *s_base = base;
+    if (tile == ntiles - 1) {
+        *a.sp.n_out_dev = base + local;
+        if (base + local > a.sp.out_cap) atomicOr(a.status, ST_FLAG_CAPACITY);
+    }
+}
+
+// Run by warp 0 after the tile's counts are in cnt: cp_tile_scan, then the
+// look-back over the earlier tiles for the tile's output offset, left in *s_base.
 // The last tile stores the total kept count.
 template <int ITEMS>
 __device__ __forceinline__ void cp_tile_offsets(const CpArgs& a, uint32_t tile, uint32_t ntiles,
                                                 uint32_t (*cnt)[CP_NW], ull* s_base) {
     const uint32_t local = cp_tile_scan<ITEMS>(cnt);
+    const ull excl = warp_look_back(a.lookback, tile, local, a.status);
     if ((threadIdx.x & 31) != 0) return;
-    ull* my = a.lookback + tile;
-    ull excl = 0;
-    if (tile == 0) {
-        *reinterpret_cast<volatile ull*>(my) = LB_INC | local;
-    } else {
-        *reinterpret_cast<volatile ull*>(my) = LB_AGG | local;
-        // Look back LB_WINDOW words per round trip: sum aggregates until an
-        // inclusive prefix.
-        int64_t t = (int64_t)tile - 1;
-        uint32_t spins = 0;
-        while (t >= 0) {
-            const int cnt_w = (t + 1) < LB_WINDOW ? (int)(t + 1) : LB_WINDOW;
-            ull v[LB_WINDOW];
-#pragma unroll
-            for (int i = 0; i < LB_WINDOW; ++i) v[i] = i < cnt_w ? ld_volatile(a.lookback + (t - i)) : 0ull;
-            int used = 0;
-            bool done = false, stalled = false;
-#pragma unroll
-            for (int i = 0; i < LB_WINDOW; ++i) {
-                if (done || stalled || i >= cnt_w) continue;
-                const ull st = v[i] >> 62;
-                if (st == 0) {
-                    stalled = true;
-                    continue;
-                }
-                excl += v[i] & LB_VAL;
-                ++used;
-                if (st == 2) done = true;
-            }
-            if (done) break;
-            t -= used;
-            if (stalled) {
-                if (++spins > SPIN_LIMIT) {
-                    atomicOr(a.status, ST_FLAG_TIMEOUT);
-                    break;
-                }
-                if (spins > 4) __nanosleep(64);
-            }
-        }
-        *reinterpret_cast<volatile ull*>(my) = LB_INC | (excl + local);
-    }
     *s_base = excl;
     if (tile == ntiles - 1) {
         const ull total = excl + local;
@@ -226,8 +221,9 @@ __device__ __forceinline__ void cp_tile_offsets(const CpArgs& a, uint32_t tile, 
 // STAGED: every thread first issues asynchronous copies of its rows of every
 // output column into shared memory, so the column reads are in flight while
 // the predicate is evaluated and the tile's offset is looked back; the
-// scatter then reads them back (each thread only its own rows).
-template <bool STAGED>
+// scatter then reads them back (each thread only its own rows). TWO: the
+// two-pass form's second pass, as below.
+template <bool STAGED, bool TWO>
 __global__ void __launch_bounds__(CP_BLOCK) compact_kernel(const __grid_constant__ CpArgs a) {
     constexpr int CP_ITEMS = STAGED ? CP_ITEMS_STAGED : CP_ITEMS_DIRECT;
     constexpr int CP_TILE = CP_BLOCK * CP_ITEMS;
@@ -238,7 +234,7 @@ __global__ void __launch_bounds__(CP_BLOCK) compact_kernel(const __grid_constant
     const CompactSpec& sp = a.sp;
     const uint64_t n = sp.n;
     const uint32_t ntiles = (uint32_t)((n + CP_TILE - 1) / CP_TILE);
-    if (threadIdx.x == 0) s_tile = atomicAdd(a.tile_ctr, 1u);
+    if (threadIdx.x == 0) s_tile = TWO ? blockIdx.x : atomicAdd(a.tile_ctr, 1u);
     __syncthreads();
     const uint32_t tile = s_tile;
     if (tile >= ntiles) return;
@@ -259,6 +255,8 @@ __global__ void __launch_bounds__(CP_BLOCK) compact_kernel(const __grid_constant
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
 
+    ull tbase0 = 0;
+    if (TWO && w == 0) tbase0 = cp_two_base(a, tile, ntiles, nullptr);
     uint32_t keep = 0;  // bit j: element base + j*BLOCK + tid is kept
 #pragma unroll
     for (int j = 0; j < CP_ITEMS; ++j) {
@@ -266,16 +264,21 @@ __global__ void __launch_bounds__(CP_BLOCK) compact_kernel(const __grid_constant
         bool k = e < n;
         if (k) {
             if (sp.mask) k = sp.mask[e] != 0;
-            if (sp.keep_valid_of) k = k && bit_valid(sp.keep_valid_of, sp.ids_in ? (uint64_t)sp.ids_in[e] : e);
+            if (sp.keep_valid_of) k = k && bit_valid(sp.keep_valid_of, e);
             for (int q = 0; q < sp.n_pred; ++q) k = k && cp_pred(sp.pred[q], e);
-            if (sp.invert) k = !k;
         }
         const uint32_t b = __ballot_sync(0xffffffffu, k && e < n);
         if (lane == 0) cnt[j][w] = __popc(b);
         if (k && e < n) keep |= 1u << j;
     }
     __syncthreads();
-    if (w == 0) cp_tile_offsets<CP_ITEMS>(a, tile, ntiles, cnt, &s_base);
+    if (w == 0) {
+        if (TWO) {
+            cp_two_offsets<CP_ITEMS>(a, tile, ntiles, cnt, tbase0, &s_base);
+        } else {
+            cp_tile_offsets<CP_ITEMS>(a, tile, ntiles, cnt, &s_base);
+        }
+    }
     __syncthreads();
     if (STAGED) asm volatile("cp.async.wait_all;" ::: "memory");
     const ull tbase = s_base;
@@ -320,13 +323,13 @@ __global__ void __launch_bounds__(CP_BLOCK) compact_kernel(const __grid_constant
         for (int j = 0; j < CP_ITEMS; ++j) {
             if (pos[j] == ~0ull) continue;
             const uint64_t e = base + (uint64_t)j * CP_BLOCK + threadIdx.x;
-            sp.row_ids[pos[j]] = (sp.ids_in ? sp.ids_in[e] : (uint32_t)e) + sp.row_id_base;
+            sp.row_ids[pos[j]] = (uint32_t)e + sp.row_id_base;
         }
     }
 }
 
 // Bulk-staged compaction (every column starts on a 16-byte boundary; no
-// ids_in / keep_valid_of selection). Thread 0 issues one bulk copy per
+// keep_valid_of selection). Thread 0 issues one bulk copy per
 // column of the tile's TILE rows (TILE * width bytes, a multiple of 16) into
 // shared memory, completing on one mbarrier; the last, partial tile is
 // copied element by element instead. Ranking, look-back and scatter follow
@@ -356,6 +359,7 @@ __global__ void __launch_bounds__(CP_BLOCK) compact_bulk_kernel(const __grid_con
     const uint32_t rows = (n - base) < (uint64_t)TILE ? (uint32_t)(n - base) : (uint32_t)TILE;
     const bool whole = rows == (uint32_t)TILE;
     bool ok = true;
+    ull tbase0 = 0;
     if (whole) {
         if (threadIdx.x == 0) {
             mbar_arrive_expect_tx(&bar, (uint32_t)TILE * a.row_w);
@@ -365,6 +369,10 @@ __global__ void __launch_bounds__(CP_BLOCK) compact_bulk_kernel(const __grid_con
                 bulk_load(stg + a.soff[c], static_cast<const unsigned char*>(sp.col[c].in) + base * wd,
                           (uint32_t)TILE * wd, &bar, pol);
             }
+        }
+        if (TWO && w == 0) {
+            __syncwarp();
+            tbase0 = cp_two_base(a, tile, ntiles, nullptr);
         }
         ok = mbar_wait(&bar, 0);
     } else {
@@ -378,6 +386,7 @@ __global__ void __launch_bounds__(CP_BLOCK) compact_bulk_kernel(const __grid_con
                 else reinterpret_cast<ulonglong2*>(dst)[i] = __ldg(reinterpret_cast<const ulonglong2*>(src) + i);
             }
         }
+        if (TWO && w == 0) tbase0 = cp_two_base(a, tile, ntiles, nullptr);
         __syncthreads();
     }
     if (!ok && threadIdx.x == 0) atomicOr(a.status, ST_FLAG_TIMEOUT);
@@ -393,7 +402,6 @@ __global__ void __launch_bounds__(CP_BLOCK) compact_bulk_kernel(const __grid_con
         if (k) {
             if (sp.mask) k = sp.mask[e] != 0;
             for (int q = 0; q < sp.n_pred; ++q) k = k && cp_pred_staged(sp.pred[q], stg + a.soff[sp.pred[q].col_idx], i, e);
-            if (sp.invert) k = !k;
         }
         k = k && ok && i < rows;
         const uint32_t b = __ballot_sync(0xffffffffu, k);
@@ -403,8 +411,7 @@ __global__ void __launch_bounds__(CP_BLOCK) compact_bulk_kernel(const __grid_con
     __syncthreads();
     if (w == 0) {
         if (TWO) {
-            cp_tile_scan<ITEMS>(cnt);
-            if (lane == 0) s_base = a.tile_off[tile];
+            cp_two_offsets<ITEMS>(a, tile, ntiles, cnt, tbase0, &s_base);
         } else {
             cp_tile_offsets<ITEMS>(a, tile, ntiles, cnt, &s_base);
         }
@@ -549,10 +556,7 @@ __global__ void __launch_bounds__(CP_BLOCK) compact_count_kernel(const __grid_co
         }
 #pragma unroll
         for (int j = 0; j < R; ++j) {
-            const uint64_t e = base + (uint64_t)j * CP_BLOCK + threadIdx.x;
-            bool k = (keep >> j) & 1u;
-            if (sp.invert && e < n) k = !k;
-            c[j / ITEMS] += __popc(__ballot_sync(0xffffffffu, k));
+            c[j / ITEMS] += __popc(__ballot_sync(0xffffffffu, (keep >> j) & 1u));
         }
         if (lane == 0) {
 #pragma unroll
@@ -570,56 +574,133 @@ __global__ void __launch_bounds__(CP_BLOCK) compact_count_kernel(const __grid_co
     }
 }
 
-// Two-pass form: one CTA turns the tile counts into exclusive output
-// offsets (SCAN_ITEMS consecutive counts per thread per round), stores the
-// total and flags a total beyond the output capacity.
-constexpr int SCAN_ITEMS = 16;
+// Two-pass form: CTA g turns the counts of tiles [g * SCAN_TILES, ...) into
+// exclusive offsets within the group, in place, and stores the group's total;
+// the scatter pass adds up the earlier groups' totals itself (24 of them for
+// 100M rows). One CTA over all 98K counts took 84 us.
 __global__ void __launch_bounds__(1024) compact_scan_kernel(const __grid_constant__ CpArgs a, uint32_t ntiles) {
-    __shared__ ull wsum[32];
-    __shared__ ull carry;
+    __shared__ uint32_t wsum[32];
     const int t = threadIdx.x, w = t >> 5, lane = t & 31;
-    if (t == 0) carry = 0;
+    const uint64_t i = (uint64_t)blockIdx.x * SCAN_TILES + 4 * (uint64_t)t;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (i + 4 <= ntiles) {
+        v = *reinterpret_cast<const uint4*>(a.tile_cnt + i);
+    } else {
+        if (i < ntiles) v.x = a.tile_cnt[i];
+        if (i + 1 < ntiles) v.y = a.tile_cnt[i + 1];
+        if (i + 2 < ntiles) v.z = a.tile_cnt[i + 2];
+    }
+    const uint32_t mine = v.x + v.y + v.z + v.w;
+    uint32_t x = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[w] = x;
     __syncthreads();
-    for (uint64_t b = 0; b < ntiles; b += 1024 * SCAN_ITEMS) {
-        const uint64_t i0 = b + (uint64_t)t * SCAN_ITEMS;
-        uint32_t v[SCAN_ITEMS];
-        ull mine = 0;
+    const uint32_t ws = wsum[lane];
+    const uint32_t before = __reduce_add_sync(0xffffffffu, lane < w ? ws : 0u);
+    const uint32_t o0 = before + x - mine, o1 = o0 + v.x, o2 = o1 + v.y, o3 = o2 + v.z;
+    if (i + 4 <= ntiles) {
+        *reinterpret_cast<uint4*>(a.tile_cnt + i) = make_uint4(o0, o1, o2, o3);
+    } else {
+        if (i < ntiles) a.tile_cnt[i] = o0;
+        if (i + 1 < ntiles) a.tile_cnt[i + 1] = o1;
+        if (i + 2 < ntiles) a.tile_cnt[i + 2] = o2;
+    }
+    if (t == 1023) a.group_tot[blockIdx.x] = o3 + v.w;
+}
+
+// NULL split: the rows' ids (ids_in[e], or e) parted into the valid ones and
+// the NULL ones, each in input order. The validity bits of permuted rows are
+// random bytes of the bitmap, which is what a split waits for, so they are
+// gathered once: this pass packs them in element order and counts each
+// 2,048-row tile's, and split_write_kernel places both parts from the packed
+// bits. (Two compactions, each gathering in both of its passes: 257 us for
+// 10M rows.)
+__global__ void __launch_bounds__(CP_BLOCK) split_count_kernel(const __grid_constant__ CpArgs a, const uint32_t* ids_in,
+                                                               uint32_t* bits) {
+    constexpr int TILE = CP_BLOCK * CP_ITEMS_DIRECT;
+    __shared__ uint32_t wcnt[CP_NW];
+    const CompactSpec& sp = a.sp;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint64_t base = (uint64_t)blockIdx.x * TILE;
+    uint32_t id[CP_ITEMS_DIRECT];
 #pragma unroll
-        for (int k = 0; k < SCAN_ITEMS; ++k) {
-            v[k] = i0 + k < ntiles ? a.tile_cnt[i0 + k] : 0u;
-            mine += v[k];
-        }
-        ull x = mine;
+    for (int j = 0; j < CP_ITEMS_DIRECT; ++j) {
+        const uint64_t e = base + (uint64_t)j * CP_BLOCK + threadIdx.x;
+        id[j] = e < sp.n ? (ids_in ? __ldg(ids_in + e) : (uint32_t)e) : 0u;
+    }
+    uint32_t c = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const ull y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) wsum[w] = x;
-        __syncthreads();
-        if (w == 0) {
-            ull ws = wsum[lane];
+    for (int j = 0; j < CP_ITEMS_DIRECT; ++j) {
+        const uint64_t e = base + (uint64_t)j * CP_BLOCK + threadIdx.x;
+        const uint32_t m = __ballot_sync(0xffffffffu, e < sp.n && bit_valid(sp.keep_valid_of, id[j]));
+        if (lane == 0) bits[e >> 5] = m;  // (whole tiles of words are allocated)
+        c += __popc(m);
+    }
+    if (lane == 0) wcnt[w] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t t = 0;
+#pragma unroll
+        for (int i = 0; i < CP_NW; ++i) t += wcnt[i];
+        a.tile_cnt[blockIdx.x] = t;
+    }
+}
+
+// sp.row_ids receives the valid ids; `nulls` the others, from row 0
+// (nulls_first) or from the number of valid rows.
+__global__ void __launch_bounds__(CP_BLOCK) split_write_kernel(const __grid_constant__ CpArgs a, const uint32_t* ids_in,
+                                                               const uint32_t* bits, uint32_t* nulls, int nulls_first, uint32_t ntiles) {
+    constexpr int TILE = CP_BLOCK * CP_ITEMS_DIRECT, WORDS = TILE / 32;
+    __shared__ uint32_t word[WORDS], pre[WORDS];
+    __shared__ ull s_base, s_total;
+    const CompactSpec& sp = a.sp;
+    const int lane = threadIdx.x & 31;
+    const uint32_t tile = blockIdx.x;
+    const uint64_t base = (uint64_t)tile * TILE;
+    if (threadIdx.x < 32) {
+        ull total;
+        const ull b = cp_two_base(a, tile, ntiles, &total);
+        uint32_t run = 0;
+#pragma unroll
+        for (int h = 0; h < WORDS; h += 32) {
+            const uint32_t m = bits[base / 32 + h + lane], c = __popc(m);
+            uint32_t x = c;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const ull y = __shfl_up_sync(0xffffffffu, ws, o);
-                if (lane >= o) ws += y;
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
             }
-            wsum[lane] = ws;  // inclusive over warps
+            word[h + lane] = m;
+            pre[h + lane] = run + x - c;
+            run += __shfl_sync(0xffffffffu, x, 31);
         }
-        __syncthreads();
-        ull run = carry + (w ? wsum[w - 1] : 0ull) + x - mine;
-#pragma unroll
-        for (int k = 0; k < SCAN_ITEMS; ++k) {
-            if (i0 + k < ntiles) a.tile_off[i0 + k] = run;
-            run += v[k];
+        if (lane == 0) {
+            s_base = b;
+            s_total = total;
+            if (tile == 0) *sp.n_out_dev = total;
         }
-        __syncthreads();
-        if (t == 0) carry += wsum[31];
-        __syncthreads();
     }
-    if (t == 0) {
-        *a.sp.n_out_dev = carry;
-        if (carry > a.sp.out_cap) atomicOr(a.status, ST_FLAG_CAPACITY);
+    uint32_t id[CP_ITEMS_DIRECT];
+#pragma unroll
+    for (int j = 0; j < CP_ITEMS_DIRECT; ++j) {
+        const uint64_t e = base + (uint64_t)j * CP_BLOCK + threadIdx.x;
+        id[j] = e < sp.n ? (ids_in ? __ldg(ids_in + e) : (uint32_t)e) : 0u;
+    }
+    __syncthreads();
+    const ull nb = nulls_first ? 0ull : s_total;
+#pragma unroll
+    for (int j = 0; j < CP_ITEMS_DIRECT; ++j) {
+        const uint32_t i = (uint32_t)j * CP_BLOCK + threadIdx.x;
+        const uint64_t e = base + i;
+        if (e >= sp.n) continue;
+        const uint32_t m = word[i >> 5];
+        const ull rank = s_base + pre[i >> 5] + __popc(m & lanemask_lt());
+        if ((m >> lane) & 1u) sp.row_ids[rank] = id[j];
+        else nulls[nb + (e - rank)] = id[j];
     }
 }
 
@@ -639,9 +720,9 @@ bolt_status compact_enqueue(bolt_ctx* ctx, cudaStream_t s, const CompactSpec& sp
     }
     a.row_w = row_w;
     // Bulk-staged tiles: columns on 16-byte boundaries, a tile of them within
-    // the stage budget, and a plain selection (no ids_in / keep_valid_of).
+    // the stage budget, and a plain selection (no keep_valid_of).
     int bulk_items = 0;
-    if (aligned && al16 && !spec.ids_in && !spec.keep_valid_of && !(flags & BOLT_FLAG_KERNEL_REGS)) {
+    if (aligned && al16 && !spec.keep_valid_of && !(flags & BOLT_FLAG_KERNEL_REGS)) {
         if (row_w * (uint32_t)(CP_BLOCK * CB_ITEMS_NARROW) <= CB_STAGE_MAX) bulk_items = CB_ITEMS_NARROW;
         else if (row_w * (uint32_t)(CP_BLOCK * CB_ITEMS_WIDE) <= CB_STAGE_MAX) bulk_items = CB_ITEMS_WIDE;
     }
@@ -659,12 +740,13 @@ bolt_status compact_enqueue(bolt_ctx* ctx, cudaStream_t s, const CompactSpec& sp
     const uint64_t ntiles = (spec.n + tile_rows - 1) / tile_rows;
     // Large bulk-staged inputs run the two-pass form (no CTA waits on
     // another); the rest run one pass with decoupled look-back.
-    const bool two = bulk_items && spec.n >= CB_TWO_PASS_ROWS;
+    const bool two = spec.n >= (bulk_items ? CB_TWO_PASS_ROWS : CP_TWO_PASS_ROWS) && !staged && !spec.keep_valid_of;
     a.tile_ctr = (uint32_t*)arena_alloc(ctx, 64);
     if (two) {
-        a.tile_cnt = (uint32_t*)arena_alloc(ctx, ntiles * 4);
-        a.tile_off = (ull*)arena_alloc(ctx, ntiles * 8);
-        if (!a.tile_cnt || !a.tile_off || !a.tile_ctr) return fail(ctx, BOLT_ERR_CAPACITY, "compaction: scratch arena too small");
+        const uint64_t groups = (ntiles + SCAN_TILES - 1) / SCAN_TILES;
+        a.group_tot = (ull*)arena_alloc(ctx, (groups + 1) * 8 + ntiles * 4);
+        a.tile_cnt = reinterpret_cast<uint32_t*>(a.group_tot + ((groups + 1) & ~1ull));
+        if (!a.group_tot || !a.tile_ctr) return fail(ctx, BOLT_ERR_CAPACITY, "compaction: scratch arena too small");
     } else {
         a.lookback = (ull*)arena_alloc(ctx, (ntiles + 1) * 8);
         if (!a.lookback || !a.tile_ctr) return fail(ctx, BOLT_ERR_CAPACITY, "compaction: scratch arena too small");
@@ -684,21 +766,26 @@ bolt_status compact_enqueue(bolt_ctx* ctx, cudaStream_t s, const CompactSpec& sp
     if (two) {
         const uint64_t ngroups = (ntiles + CC_GROUP - 1) / CC_GROUP;
         const unsigned cg = (unsigned)std::min<uint64_t>(ngroups, (uint64_t)ctx->num_sms * 8);
+        const unsigned sgrid = (unsigned)((ntiles + SCAN_TILES - 1) / SCAN_TILES);
         // Vectorised count: a byte mask or one Int32 conjunct without a
         // validity bitmap, on 16-byte boundaries (1,024-row tiles only).
-        const bool vec = bulk_items == 4 && !spec.invert &&
+        const bool vec = bulk_items == 4 &&
                          ((spec.mask && spec.n_pred == 0 && reinterpret_cast<uintptr_t>(spec.mask) % 16 == 0) ||
                           (!spec.mask && spec.n_pred == 1 && spec.pred[0].dtype == BOLT_I32 && !spec.pred[0].valid &&
                            reinterpret_cast<uintptr_t>(spec.pred[0].col) % 16 == 0));
-        if (bulk_items == CB_ITEMS_NARROW) {
+        if (!bulk_items) {
+            compact_count_kernel<CP_ITEMS_DIRECT, false><<<cg, CP_BLOCK, 0, s>>>(a);
+            compact_scan_kernel<<<sgrid, 1024, 0, s>>>(a, (uint32_t)ntiles);
+            compact_kernel<false, true><<<(unsigned)ntiles, CP_BLOCK, 0, s>>>(a);
+        } else if (bulk_items == CB_ITEMS_NARROW) {
             if (vec) compact_count_kernel<CB_ITEMS_NARROW, true><<<cg, CP_BLOCK, 0, s>>>(a);
             else compact_count_kernel<CB_ITEMS_NARROW, false><<<cg, CP_BLOCK, 0, s>>>(a);
-            compact_scan_kernel<<<1, 1024, 0, s>>>(a, (uint32_t)ntiles);
+            compact_scan_kernel<<<sgrid, 1024, 0, s>>>(a, (uint32_t)ntiles);
             BOLT_CUDA(ctx, smem_optin(compact_bulk_kernel<CB_ITEMS_NARROW, true>, ctx));
             compact_bulk_kernel<CB_ITEMS_NARROW, true><<<(unsigned)ntiles, CP_BLOCK, stage_bytes, s>>>(a);
         } else {
             compact_count_kernel<CB_ITEMS_WIDE, false><<<cg, CP_BLOCK, 0, s>>>(a);
-            compact_scan_kernel<<<1, 1024, 0, s>>>(a, (uint32_t)ntiles);
+            compact_scan_kernel<<<sgrid, 1024, 0, s>>>(a, (uint32_t)ntiles);
             BOLT_CUDA(ctx, smem_optin(compact_bulk_kernel<CB_ITEMS_WIDE, true>, ctx));
             compact_bulk_kernel<CB_ITEMS_WIDE, true><<<(unsigned)ntiles, CP_BLOCK, stage_bytes, s>>>(a);
         }
@@ -710,13 +797,41 @@ bolt_status compact_enqueue(bolt_ctx* ctx, cudaStream_t s, const CompactSpec& sp
         BOLT_CUDA(ctx, smem_optin(compact_bulk_kernel<CB_ITEMS_WIDE, false>, ctx));
         compact_bulk_kernel<CB_ITEMS_WIDE, false><<<(unsigned)ntiles, CP_BLOCK, stage_bytes, s>>>(a);
     } else if (staged) {
-        BOLT_CUDA(ctx, smem_optin(compact_kernel<true>, ctx));
-        compact_kernel<true><<<(unsigned)ntiles, CP_BLOCK, stage_bytes, s>>>(a);
+        BOLT_CUDA(ctx, smem_optin(compact_kernel<true, false>, ctx));
+        compact_kernel<true, false><<<(unsigned)ntiles, CP_BLOCK, stage_bytes, s>>>(a);
     } else {
-        compact_kernel<false><<<(unsigned)ntiles, CP_BLOCK, 0, s>>>(a);
+        compact_kernel<false, false><<<(unsigned)ntiles, CP_BLOCK, 0, s>>>(a);
     }
     kernel_mark_end(ctx, flags, s);
     ctx->last_launches++;
+    BOLT_CUDA(ctx, cudaGetLastError());
+    return BOLT_OK;
+}
+
+bolt_status null_split_enqueue(bolt_ctx* ctx, cudaStream_t s, uint64_t n, const uint8_t* valid, const uint32_t* ids_in,
+                               uint32_t* valid_ids, uint32_t* nulls, bool nulls_first, ull* n_valid_dev) {
+    CpArgs a{};
+    a.sp.n = n;
+    a.sp.keep_valid_of = valid;
+    a.sp.row_ids = valid_ids;
+    a.sp.n_out_dev = n_valid_dev;
+    a.status = ctx->d_status;
+    if (n == 0) {
+        BOLT_CUDA(ctx, cudaMemsetAsync(n_valid_dev, 0, 8, s));
+        return BOLT_OK;
+    }
+    constexpr uint64_t TILE = (uint64_t)CP_BLOCK * CP_ITEMS_DIRECT;
+    const uint64_t ntiles = (n + TILE - 1) / TILE, groups = (ntiles + SCAN_TILES - 1) / SCAN_TILES;
+    const uint64_t mark = ctx->arena_used;  // (scratch of these launches only: later work on the stream may reuse it)
+    a.group_tot = (ull*)arena_alloc(ctx, (groups + 1) * 8 + ntiles * 4);
+    a.tile_cnt = reinterpret_cast<uint32_t*>(a.group_tot + ((groups + 1) & ~1ull));
+    uint32_t* bits = (uint32_t*)arena_alloc(ctx, ntiles * TILE / 8);
+    if (!a.group_tot || !bits) return fail(ctx, BOLT_ERR_CAPACITY, "NULL split: scratch arena too small");
+    split_count_kernel<<<(unsigned)ntiles, CP_BLOCK, 0, s>>>(a, ids_in, bits);
+    compact_scan_kernel<<<(unsigned)groups, 1024, 0, s>>>(a, (uint32_t)ntiles);
+    split_write_kernel<<<(unsigned)ntiles, CP_BLOCK, 0, s>>>(a, ids_in, bits, nulls, nulls_first ? 1 : 0, (uint32_t)ntiles);
+    ctx->arena_used = mark;
+    ctx->last_launches += 3;
     BOLT_CUDA(ctx, cudaGetLastError());
     return BOLT_OK;
 }

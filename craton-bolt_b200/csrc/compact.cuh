@@ -31,9 +31,7 @@ struct CompactSpec {
     CompactPred pred[CP_MAX_PREDS];
     int32_t n_pred = 0;
     const uint8_t* mask = nullptr;          // byte mask (keep when != 0)
-    const uint8_t* keep_valid_of = nullptr; // keep rows whose bit is set (or clear, see invert)
-    const uint32_t* ids_in = nullptr;       // element e stands for row ids_in[e] (validity test, row ids)
-    int32_t invert = 0;                     // keep the complement of the selection
+    const uint8_t* keep_valid_of = nullptr; // keep rows whose bit is set
     CompactCol col[CP_MAX_COLS];
     int32_t n_cols = 0;
     uint32_t* row_ids = nullptr;            // selected row indices (+ row_id_base)
@@ -45,5 +43,12 @@ struct CompactSpec {
 // Enqueues one fused predicate-evaluation + scan + scatter pass.
 // flags: BOLT_FLAG_PROFILE records the kernel's device time.
 bolt_status compact_enqueue(bolt_ctx* ctx, cudaStream_t s, const CompactSpec& spec, uint32_t flags = 0);
+
+// Parts the rows (ids_in[e] for e in [0, n), or e itself) by their validity
+// bit, each part in input order: the valid ids to valid_ids, the NULL ones to
+// nulls[0..) (nulls_first) or nulls[number of valid rows..). n_valid_dev
+// receives the number of valid rows.
+bolt_status null_split_enqueue(bolt_ctx* ctx, cudaStream_t s, uint64_t n, const uint8_t* valid, const uint32_t* ids_in,
+                               uint32_t* valid_ids, uint32_t* nulls, bool nulls_first, ull* n_valid_dev);
 
 }  // namespace bolt

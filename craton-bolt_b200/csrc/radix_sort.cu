@@ -48,8 +48,8 @@ constexpr int SORT_BLOCK = 256;
 constexpr int SORT_ITEMS_32 = 20;
 constexpr int SORT_ITEMS_64 = 16;
 constexpr int SORT_TILE_MIN = SORT_BLOCK * SORT_ITEMS_64;
-constexpr int HIST_CHUNK = 8192;
-constexpr int HIST_BLOCK = 512;
+constexpr int HIST_CHUNK = 4096;
+constexpr int HIST_BLOCK = 256;
 constexpr uint32_t LB_AGG = 1u << 30;
 constexpr uint32_t LB_INC = 2u << 30;
 constexpr uint32_t LB_VAL = (1u << 30) - 1;
@@ -196,8 +196,8 @@ __device__ __forceinline__ uint64_t seg_n(const SegDesc& d) {
 
 // Digit histograms of every segment. Bound by its shared-memory counter adds
 // (one per digit and key, about 7.5 lanes per SM and cycle; four copies of
-// every counter in neighbouring banks changed nothing). A CTA takes
-// neighbouring items and flushes its counters once per segment.
+// every counter in neighbouring banks changed nothing). A CTA flushes its
+// counters once per segment it meets.
 template <typename K>
 __global__ void __launch_bounds__(HIST_BLOCK) sort_hist_kernel(SortArgs a) {
     constexpr int NP = KeyTraits<K>::NPASS;
@@ -218,10 +218,7 @@ __global__ void __launch_bounds__(HIST_BLOCK) sort_hist_kernel(SortArgs a) {
             if (c) atomicAdd(&gh[i], c);
         }
     };
-    const uint32_t per = (a.total_hist_items + gridDim.x - 1) / gridDim.x;
-    const uint32_t first = blockIdx.x * per;
-    const uint32_t stop = min(first + per, a.total_hist_items);
-    for (uint32_t item = first; item < stop; ++item) {
+    for (uint32_t item = blockIdx.x; item < a.total_hist_items; item += gridDim.x) {
         const int sg = seg_of(a.hist_begins, a.nseg, item);
         if (sg != cur) {
             if (cur >= 0) flush();
@@ -1195,7 +1192,7 @@ bolt_status run_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
     if (nseg == 0) return BOLT_OK;
     std::vector<SegDesc> segs(nseg);
     std::vector<uint32_t> begins(3 * (nseg + 1));
-    uint64_t total_n = 0, items = 0, hitems = 0, litems = 0;
+    uint64_t total_n = 0, end_n = 0, items = 0, hitems = 0, litems = 0;
     // Rows of one local work item: a few chunks, so that finding its ends is
     // a small part of it, but enough items for every CTA.
     uint64_t sum_n = 0;
@@ -1211,6 +1208,7 @@ bolt_status run_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
         begins[i] = (uint32_t)items;
         begins[nseg + 1 + i] = (uint32_t)hitems;
         begins[2 * (nseg + 1) + i] = (uint32_t)litems;
+        end_n = total_n + g.n;
         total_n += (g.n + 15) & ~15ull;  // (16-byte aligned buffers for the local step's prefetches)
         items += (g.n + SORT_TILE - 1) / SORT_TILE;
         hitems += (g.n + HIST_CHUNK - 1) / HIST_CHUNK;
@@ -1232,7 +1230,7 @@ bolt_status run_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
     a.total_loc_items = (uint32_t)litems;
     a.loc_range = (uint32_t)loc_range;
     a.lb_stride = items * 256;
-    const uint64_t nb = total_n ? total_n : 1;
+    const uint64_t nb = end_n ? end_n : 1;
     SegDesc* d_segs = (SegDesc*)arena_alloc(ctx, sizeof(SegDesc) * nseg);
     uint32_t* d_begins = (uint32_t*)arena_alloc(ctx, 4 * begins.size());
     a.kA = arena_alloc(ctx, nb * sizeof(K));
@@ -1257,7 +1255,7 @@ bolt_status run_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
     st = stage_upload(ctx, s, d_begins, begins.data(), 4 * begins.size());
     if (st != BOLT_OK) return st;
     BOLT_CUDA(ctx, cudaMemsetAsync(a.hist, 0, (uint64_t)nseg * NP * 256 * 4, s));
-    const unsigned hb = (unsigned)std::min<uint64_t>(hitems, (uint64_t)ctx->num_sms * 4);
+    const unsigned hb = (unsigned)std::min<uint64_t>(hitems, (uint64_t)ctx->num_sms * 8);
     sort_hist_kernel<K><<<hb, HIST_BLOCK, 0, s>>>(a);
     BOLT_CUDA(ctx, smem_optin(sort_plan_kernel<K>, ctx));
     sort_plan_kernel<K><<<nseg, PLAN_BLOCK, 2 * PLAN_SAMPLES * 8, s>>>(a);
@@ -1371,23 +1369,12 @@ extern "C" bolt_status bolt_radix_sort_perm_multi(bolt_ctx* ctx, const bolt_col_
             // their current relative order and go first or last.
             uint32_t* valid_ids = (uint32_t*)arena_alloc(ctx, (n ? n : 1) * 4);
             if (!valid_ids) return fail(ctx, BOLT_ERR_CAPACITY, "ORDER BY: scratch arena too small");
-            CompactSpec cv;
-            cv.n = n;
-            cv.keep_valid_of = key.validity;
-            cv.ids_in = cur;
-            cv.row_ids = valid_ids;
-            cv.n_out_dev = cnt;
-            st = compact_enqueue(ctx, s, cv);
+            st = null_split_enqueue(ctx, s, n, key.validity, cur, valid_ids, dst, nulls_first[k] != 0, cnt);
             if (st != BOLT_OK) return st;
             BOLT_CUDA(ctx, cudaMemcpyAsync(ctx->h_words, cnt, 8, cudaMemcpyDeviceToHost, s));
             BOLT_CUDA(ctx, cudaStreamSynchronize(s));
             const ull nv = ctx->h_words[0];
             const uint64_t nn = n - nv;
-            CompactSpec cn = cv;
-            cn.invert = 1;
-            cn.row_ids = dst + (nulls_first[k] ? 0 : nv);
-            st = compact_enqueue(ctx, s, cn);
-            if (st != BOLT_OK) return st;
             seg.payload_in = valid_ids;
             sp.indirect = 1;
             seg.n = nv;
