@@ -13,8 +13,8 @@
 //      (cmp_tuple, groupby_wide.rs:410);
 //   3. run starts are marked and compacted: start g is group g's first
 //      position, and the number of starts is the group count;
-//   4. one warp per group folds each aggregate over the group's rows in row
-//      order, so every result equals the reference's sequential fold bit for
+//   4. one thread (short groups) or one warp (longer ones) per group folds
+//      each aggregate over the group's rows in row order, so every result equals the reference's sequential fold bit for
 //      bit: SUM over integers wraps in i64 (groupby_wide.rs:695-705), SUM and
 //      AVG over floats add in f64, MIN / MAX keep the first valid value and
 //      replace it only when x < v / x > v (a NaN never replaces a value, a
@@ -79,18 +79,30 @@ __global__ void __launch_bounds__(256) wide_valid_kernel(const uint8_t* v0, cons
         flag[i] = (bit_valid(v0, i) && bit_valid(v1, i)) ? 1 : 0;
 }
 
-// flag[i] = 1 when sorted position i starts a run of equal (key0, key1).
+// flag[i] = 1 when sorted position i starts a run of equal (key0, key1). The
+// keys are gathered at random rows: each lane gathers its own row's and takes
+// the previous row's from its neighbour. Bound by those reads, a 128-byte
+// line per row and key from DRAM (10M rows: 170 us; the neighbour's, in L1,
+// cost nothing either way).
 __global__ void __launch_bounds__(256) wide_mark_kernel(const void* k0, int dt0, const void* k1, int dt1,
                                                          const uint32_t* perm, uint64_t n, uint8_t* flag) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        bool start = i == 0;
-        if (!start) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); b < n; b += step) {  // (warp-uniform)
+        const uint64_t i = b + lane;
+        ll a0 = 0, a1 = 0;
+        if (i < n) {
             const uint32_t r = perm[i];
-            const uint32_t p = perm[i - 1];
-            start = wide_load_i(k0, dt0, r) != wide_load_i(k0, dt0, p) ||
-                    wide_load_i(k1, dt1, r) != wide_load_i(k1, dt1, p);
+            a0 = wide_load_i(k0, dt0, r);
+            a1 = wide_load_i(k1, dt1, r);
         }
-        flag[i] = start ? 1 : 0;
+        ll p0 = __shfl_up_sync(0xffffffffu, a0, 1), p1 = __shfl_up_sync(0xffffffffu, a1, 1);
+        if (lane == 0 && i > 0) {
+            const uint32_t p = perm[i - 1];
+            p0 = wide_load_i(k0, dt0, p);
+            p1 = wide_load_i(k1, dt1, p);
+        }
+        if (i < n) flag[i] = i == 0 || a0 != p0 || a1 != p1;
     }
 }
 
@@ -116,7 +128,103 @@ __device__ __forceinline__ WideElem wide_elem(const WideArgs& a, const WideAgg& 
     return e;
 }
 
-// One warp per group: the group's keys from its first row, then every
+// Groups up to this many rows are folded by one thread each, longer ones by
+// one warp: a warp per group of ten rows leaves two thirds of its lanes idle
+// and walks its 32 shuffles for ten values (10M rows in 1M groups: 1,290 us, a
+// thread each 263 us).
+constexpr uint64_t WIDE_THREAD_ROWS = 48;
+constexpr int WIDE_TU = 4;  // rows of a group in flight per thread
+
+// Writes aggregate q of group g (cnt valid inputs; the integer or the float
+// accumulator; seen: the group had a valid input).
+__device__ __forceinline__ void wide_store(const WideAgg& w, uint64_t g, uint64_t cnt, ull si, ll mi, double f, bool seen) {
+    bool valid = true;
+    switch (w.op) {
+    case BOLT_AGG_COUNT_STAR:
+    case BOLT_AGG_COUNT:
+        ((ll*)w.out)[g] = (ll)cnt;
+        break;
+    case BOLT_AGG_AVG:
+        valid = cnt > 0;
+        ((double*)w.out)[g] = valid ? f / (double)cnt : 0.0;
+        break;
+    default:  // SUM, MIN, MAX
+        valid = seen;
+        if (w.out_dtype == BOLT_F64) ((double*)w.out)[g] = valid ? f : 0.0;
+        else if (w.out_dtype == BOLT_F32) ((float*)w.out)[g] = valid ? (float)f : 0.0f;
+        else if (w.out_dtype == BOLT_I32) ((int32_t*)w.out)[g] = valid ? (int32_t)mi : 0;
+        else ((ll*)w.out)[g] = valid ? (w.op == BOLT_AGG_SUM ? (ll)si : mi) : 0;
+        break;
+    }
+    if (w.out_valid) set_bit_atomic(w.out_valid, g, valid);
+}
+
+// One thread per group of at most WIDE_THREAD_ROWS rows: every aggregate in
+// row order, WIDE_TU rows loaded before the first is folded.
+__global__ void __launch_bounds__(256) wide_fold_short_kernel(const __grid_constant__ WideArgs a) {
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < a.n_write; g += step) {
+        const uint64_t beg = a.starts[g];
+        const uint64_t end = g + 1 < a.n_groups ? a.starts[g + 1] : a.n_kept;
+        if (end - beg > WIDE_THREAD_ROWS) continue;
+        const uint32_t r0 = a.perm[beg];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const ll kv = wide_load_i(a.key[k], a.kdt[k], r0);
+            if (a.kdt[k] == BOLT_I32) ((int32_t*)a.out_key[k])[g] = (int32_t)kv;
+            else ((ll*)a.out_key[k])[g] = kv;
+            if (a.out_key_valid[k]) set_bit_atomic(a.out_key_valid[k], g, true);
+        }
+        for (int q = 0; q < a.n_aggs; ++q) {
+            const WideAgg& w = a.agg[q];
+            const bool sum = w.op == BOLT_AGG_SUM || w.op == BOLT_AGG_AVG, is_min = w.op == BOLT_AGG_MIN;
+            const bool value = w.op != BOLT_AGG_COUNT;
+            uint64_t cnt = 0;
+            ull si = 0;
+            ll mi = is_min ? LLONG_MAX : LLONG_MIN;
+            double f = 0.0;
+            bool seen = false;
+            if (w.op == BOLT_AGG_COUNT_STAR) {
+                cnt = end - beg;
+            } else {
+                for (uint64_t c = beg; c < end; c += WIDE_TU) {
+                    bool v[WIDE_TU];
+                    ll xi[WIDE_TU];
+                    double xf[WIDE_TU];
+#pragma unroll
+                    for (int u = 0; u < WIDE_TU; ++u) {
+                        v[u] = false;
+                        xi[u] = 0;
+                        xf[u] = 0.0;
+                        if (c + u < end) {
+                            const uint32_t r = a.perm[c + u];
+                            v[u] = bit_valid(w.in_valid, r);
+                            if (value && w.fold_f) xf[u] = wide_load_f(w.in, w.in_dtype, r);
+                            else if (value) xi[u] = wide_load_i(w.in, w.in_dtype, r);
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < WIDE_TU; ++u) {
+                        if (!v[u]) continue;
+                        ++cnt;
+                        if (!w.fold_f) {
+                            si += (ull)xi[u];
+                            mi = is_min ? (xi[u] < mi ? xi[u] : mi) : (xi[u] > mi ? xi[u] : mi);
+                        } else if (sum) {
+                            f = f + xf[u];
+                        } else if (!seen || (is_min ? xf[u] < f : xf[u] > f)) {
+                            f = xf[u];
+                        }
+                        seen = true;
+                    }
+                }
+            }
+            wide_store(w, g, cnt, si, mi, f, seen);
+        }
+    }
+}
+
+// One warp per longer group: the group's keys from its first row, then every
 // aggregate over the group's rows. Integer aggregates (wrapping SUM, COUNT,
 // MIN / MAX) do not depend on the order: each lane folds its own rows
 // (WIDE_PF chunks loaded at a time) and the warp reduces at the end. Float
@@ -127,105 +235,100 @@ __global__ void __launch_bounds__(256) wide_fold_kernel(const __grid_constant__ 
     const int lane = threadIdx.x & 31;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t n_warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t g = warp; g < a.n_write; g += n_warps) {
-        const uint64_t beg = a.starts[g];
-        const uint64_t end = g + 1 < a.n_groups ? a.starts[g + 1] : a.n_kept;
-        if (lane < 2) {
-            const ll kv = wide_load_i(a.key[lane], a.kdt[lane], a.perm[beg]);
-            if (a.kdt[lane] == BOLT_I32) ((int32_t*)a.out_key[lane])[g] = (int32_t)kv;
-            else ((ll*)a.out_key[lane])[g] = kv;
-            if (a.out_key_valid[lane]) set_bit_atomic(a.out_key_valid[lane], g, true);
+    // 32 groups at a time: one warp load of their lengths says which are long
+    // (of few groups, each warp gets one).
+    const uint64_t span = a.n_write < 32 * n_warps ? 1 : 32;
+    for (uint64_t g0 = warp * span; g0 < a.n_write; g0 += n_warps * span) {
+        bool is_long = false;
+        if ((uint64_t)lane < span && g0 + lane < a.n_write) {
+            const uint64_t gl = g0 + lane;
+            const uint64_t e = gl + 1 < a.n_groups ? a.starts[gl + 1] : a.n_kept;
+            is_long = e - a.starts[gl] > WIDE_THREAD_ROWS;
         }
-        for (int q = 0; q < a.n_aggs; ++q) {
-            const WideAgg& w = a.agg[q];
-            uint64_t cnt = 0;
-            ull si = 0;       // integer SUM (wrapping)
-            ll mi = 0;        // integer MIN / MAX
-            double f = 0.0;   // float SUM, AVG numerator, float MIN / MAX
-            bool seen = false;
-            if (w.op == BOLT_AGG_COUNT_STAR) {
-                cnt = end - beg;
-            } else if (!w.fold_f) {
-                const bool is_min = w.op == BOLT_AGG_MIN;
-                ll lm = is_min ? LLONG_MAX : LLONG_MIN;
-                bool lseen = false;
-                for (uint64_t c = beg; c < end; c += 32 * WIDE_PF) {
-                    WideElem e[WIDE_PF];  // every load of WIDE_PF chunks issued before any is used
+        uint32_t todo = __ballot_sync(0xffffffffu, is_long);
+        while (todo) {
+            const uint64_t g = g0 + (uint32_t)__ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint64_t beg = a.starts[g];
+            const uint64_t end = g + 1 < a.n_groups ? a.starts[g + 1] : a.n_kept;
+            if (lane < 2) {
+                const ll kv = wide_load_i(a.key[lane], a.kdt[lane], a.perm[beg]);
+                if (a.kdt[lane] == BOLT_I32) ((int32_t*)a.out_key[lane])[g] = (int32_t)kv;
+                else ((ll*)a.out_key[lane])[g] = kv;
+                if (a.out_key_valid[lane]) set_bit_atomic(a.out_key_valid[lane], g, true);
+            }
+            for (int q = 0; q < a.n_aggs; ++q) {
+                const WideAgg& w = a.agg[q];
+                uint64_t cnt = 0;
+                ull si = 0;       // integer SUM (wrapping)
+                ll mi = 0;        // integer MIN / MAX
+                double f = 0.0;   // float SUM, AVG numerator, float MIN / MAX
+                bool seen = false;
+                if (w.op == BOLT_AGG_COUNT_STAR) {
+                    cnt = end - beg;
+                } else if (!w.fold_f) {
+                    const bool is_min = w.op == BOLT_AGG_MIN;
+                    ll lm = is_min ? LLONG_MAX : LLONG_MIN;
+                    bool lseen = false;
+                    for (uint64_t c = beg; c < end; c += 32 * WIDE_PF) {
+                        WideElem e[WIDE_PF];  // every load of WIDE_PF chunks issued before any is used
 #pragma unroll
-                    for (int p = 0; p < WIDE_PF; ++p) e[p] = wide_elem(a, w, c + (uint64_t)p * 32 + lane, end);
+                        for (int p = 0; p < WIDE_PF; ++p) e[p] = wide_elem(a, w, c + (uint64_t)p * 32 + lane, end);
 #pragma unroll
-                    for (int p = 0; p < WIDE_PF; ++p) {
-                        cnt += (uint64_t)__popc(__ballot_sync(0xffffffffu, e[p].v));
-                        if (e[p].v) {
-                            si += (ull)e[p].xi;
-                            lm = is_min ? (e[p].xi < lm ? e[p].xi : lm) : (e[p].xi > lm ? e[p].xi : lm);
-                            lseen = true;
-                        }
-                    }
-                }
-                seen = __any_sync(0xffffffffu, lseen);
-                for (int o = 16; o > 0; o >>= 1) {
-                    si += __shfl_xor_sync(0xffffffffu, si, o);
-                    const ll y = __shfl_xor_sync(0xffffffffu, lm, o);
-                    lm = is_min ? (y < lm ? y : lm) : (y > lm ? y : lm);
-                }
-                mi = lm;
-            } else {
-                const int kind = (w.op == BOLT_AGG_SUM || w.op == BOLT_AGG_AVG) ? 0 : (w.op == BOLT_AGG_MIN ? 1 : 2);
-                // WIDE_PF chunks in flight: chunk i + WIDE_PF is loaded
-                // before chunk i is folded. Lanes past the group's end load
-                // nothing and hold no valid value.
-                WideElem buf[WIDE_PF];
-#pragma unroll
-                for (int p = 0; p < WIDE_PF; ++p) buf[p] = wide_elem(a, w, beg + (uint64_t)p * 32 + lane, end);
-                for (uint64_t c = beg; c < end; c += 32 * WIDE_PF) {
-#pragma unroll
-                    for (int p = 0; p < WIDE_PF; ++p) {
-                        const WideElem e = buf[p];
-                        buf[p] = wide_elem(a, w, c + (uint64_t)(p + WIDE_PF) * 32 + lane, end);
-                        const unsigned m = __ballot_sync(0xffffffffu, e.v);
-                        if (m == 0) continue;  // warp-uniform
-                        cnt += (uint64_t)__popc(m);
-                        if (kind == 0) {
-#pragma unroll
-                            for (int t = 0; t < 32; ++t) {
-                                const double x = __shfl_sync(0xffffffffu, e.xf, t);
-                                f = ((m >> t) & 1) ? f + x : f;
-                            }
-                        } else {
-#pragma unroll
-                            for (int t = 0; t < 32; ++t) {
-                                const double x = __shfl_sync(0xffffffffu, e.xf, t);
-                                const bool on = (m >> t) & 1;
-                                const bool take = on && (!seen || (kind == 1 ? x < f : x > f));
-                                f = take ? x : f;
-                                seen = seen || on;
+                        for (int p = 0; p < WIDE_PF; ++p) {
+                            cnt += (uint64_t)__popc(__ballot_sync(0xffffffffu, e[p].v));
+                            if (e[p].v) {
+                                si += (ull)e[p].xi;
+                                lm = is_min ? (e[p].xi < lm ? e[p].xi : lm) : (e[p].xi > lm ? e[p].xi : lm);
+                                lseen = true;
                             }
                         }
                     }
+                    seen = __any_sync(0xffffffffu, lseen);
+                    for (int o = 16; o > 0; o >>= 1) {
+                        si += __shfl_xor_sync(0xffffffffu, si, o);
+                        const ll y = __shfl_xor_sync(0xffffffffu, lm, o);
+                        lm = is_min ? (y < lm ? y : lm) : (y > lm ? y : lm);
+                    }
+                    mi = lm;
+                } else {
+                    const int kind = (w.op == BOLT_AGG_SUM || w.op == BOLT_AGG_AVG) ? 0 : (w.op == BOLT_AGG_MIN ? 1 : 2);
+                    // WIDE_PF chunks in flight: chunk i + WIDE_PF is loaded
+                    // before chunk i is folded. Lanes past the group's end load
+                    // nothing and hold no valid value.
+                    WideElem buf[WIDE_PF];
+#pragma unroll
+                    for (int p = 0; p < WIDE_PF; ++p) buf[p] = wide_elem(a, w, beg + (uint64_t)p * 32 + lane, end);
+                    for (uint64_t c = beg; c < end; c += 32 * WIDE_PF) {
+#pragma unroll
+                        for (int p = 0; p < WIDE_PF; ++p) {
+                            const WideElem e = buf[p];
+                            buf[p] = wide_elem(a, w, c + (uint64_t)(p + WIDE_PF) * 32 + lane, end);
+                            const unsigned m = __ballot_sync(0xffffffffu, e.v);
+                            if (m == 0) continue;  // warp-uniform
+                            cnt += (uint64_t)__popc(m);
+                            if (kind == 0) {
+#pragma unroll
+                                for (int t = 0; t < 32; ++t) {
+                                    const double x = __shfl_sync(0xffffffffu, e.xf, t);
+                                    f = ((m >> t) & 1) ? f + x : f;
+                                }
+                            } else {
+#pragma unroll
+                                for (int t = 0; t < 32; ++t) {
+                                    const double x = __shfl_sync(0xffffffffu, e.xf, t);
+                                    const bool on = (m >> t) & 1;
+                                    const bool take = on && (!seen || (kind == 1 ? x < f : x > f));
+                                    f = take ? x : f;
+                                    seen = seen || on;
+                                }
+                            }
+                        }
+                    }
+                    if (kind == 0) seen = cnt > 0;
                 }
-                if (kind == 0) seen = cnt > 0;
+                if (lane == 0) wide_store(w, g, cnt, si, mi, f, seen);
             }
-            if (lane != 0) continue;
-            bool valid = true;
-            switch (w.op) {
-            case BOLT_AGG_COUNT_STAR:
-            case BOLT_AGG_COUNT:
-                ((ll*)w.out)[g] = (ll)cnt;
-                break;
-            case BOLT_AGG_AVG:
-                valid = cnt > 0;
-                ((double*)w.out)[g] = valid ? f / (double)cnt : 0.0;
-                break;
-            default:  // SUM, MIN, MAX
-                valid = seen;
-                if (w.out_dtype == BOLT_F64) ((double*)w.out)[g] = valid ? f : 0.0;
-                else if (w.out_dtype == BOLT_F32) ((float*)w.out)[g] = valid ? (float)f : 0.0f;
-                else if (w.out_dtype == BOLT_I32) ((int32_t*)w.out)[g] = valid ? (int32_t)mi : 0;
-                else ((ll*)w.out)[g] = valid ? (w.op == BOLT_AGG_SUM ? (ll)si : mi) : 0;
-                break;
-            }
-            if (w.out_valid) set_bit_atomic(w.out_valid, g, valid);
         }
     }
 }
@@ -391,8 +494,13 @@ bolt_status gb_wide(bolt_ctx* ctx, const bolt_groupby_desc* d, bolt_groupby_out*
     wa.n_kept = n_kept;
     wa.n_write = std::min<uint64_t>(n_groups, out_cap);
     if (wa.n_write) {
-        const unsigned blocks = (unsigned)std::min<uint64_t>((wa.n_write + 7) / 8, (uint64_t)ctx->num_sms * 8);
-        wide_fold_kernel<<<blocks, 256, 0, s>>>(wa);
+        wide_fold_short_kernel<<<grid_for(wa.n_write, 256, ctx->num_sms * 8), 256, 0, s>>>(wa);
+        // (else no group is longer)
+        if (n_kept > WIDE_THREAD_ROWS) {
+            const unsigned blocks = (unsigned)std::min<uint64_t>((wa.n_write + 7) / 8, (uint64_t)ctx->num_sms * 8);
+            wide_fold_kernel<<<blocks, 256, 0, s>>>(wa);
+            launches += 1;
+        }
         BOLT_CUDA(ctx, cudaGetLastError());
         launches += 1;
     }
