@@ -353,6 +353,15 @@ using Spec4 = SpecK<2, K_COUNT, K_SUM_I64>;                        // COUNT, SUM
 using Spec5 = SpecK<2, K_COUNT, K_SUM_FX>;                         // COUNT, SUM f64
 using Spec6 = SpecK<1, K_COUNT>;                                   // COUNT
 using Spec7 = SpecK<2, K_COUNT, K_SUM_I32>;                        // COUNT, SUM i32
+using Spec8 = SpecK<1, K_SUM_I64>;                                 // SUM i64
+using Spec9 = SpecK<1, K_SUM_FX>;                                  // SUM f64
+using Spec10 = SpecK<1, K_SUM_I32>;                                // SUM i32
+using Spec11 = SpecK<3, K_COUNT, K_SUM_FX, K_SUM_FX>;              // COUNT, two SUM / AVG f64
+using Spec12 = SpecK<4, K_COUNT, K_SUM_FX, K_SUM_FX, K_SUM_FX>;    // COUNT, three SUM / AVG f64
+using Spec13 = SpecK<2, K_SUM_I64, K_SUM_I64>;                     // two SUM i64
+using Spec14 = SpecK<3, K_COUNT, K_COUNT, K_SUM_FX>;               // COUNT(*), nullable SUM / AVG f64
+using Spec15 = SpecK<3, K_COUNT, K_COUNT, K_SUM_I64>;              // COUNT(*), nullable SUM / AVG i64
+constexpr int GB_SPECS = 15;
 
 template <class SP>
 __device__ __forceinline__ int skind(const GbParams& p, int s) {

@@ -988,6 +988,14 @@ AggKernel agg_kernel_for(int spec, int n_st) {
     case 5: return gb_agg_kernel<4, 2, Spec5>;
     case 6: return gb_agg_kernel<4, 1, Spec6>;
     case 7: return gb_agg_kernel<4, 2, Spec7>;
+    case 8: return gb_agg_kernel<4, 1, Spec8>;
+    case 9: return gb_agg_kernel<4, 1, Spec9>;
+    case 10: return gb_agg_kernel<4, 1, Spec10>;
+    case 11: return gb_agg_kernel<4, 3, Spec11>;
+    case 12: return gb_agg_kernel<4, 4, Spec12>;
+    case 13: return gb_agg_kernel<4, 2, Spec13>;
+    case 14: return gb_agg_kernel<4, 3, Spec14>;
+    case 15: return gb_agg_kernel<4, 3, Spec15>;
     default: return n_st <= 4 ? gb_agg_kernel<4, 4, SpecGeneric> : gb_agg_kernel<2, 8, SpecGeneric>;
     }
 }
@@ -1001,6 +1009,14 @@ BatchKernel batch_kernel_for(int spec, int max_st) {
     case 5: return gb_batch_agg_kernel<4, 2, Spec5>;
     case 6: return gb_batch_agg_kernel<4, 1, Spec6>;
     case 7: return gb_batch_agg_kernel<4, 2, Spec7>;
+    case 8: return gb_batch_agg_kernel<4, 1, Spec8>;
+    case 9: return gb_batch_agg_kernel<4, 1, Spec9>;
+    case 10: return gb_batch_agg_kernel<4, 1, Spec10>;
+    case 11: return gb_batch_agg_kernel<4, 3, Spec11>;
+    case 12: return gb_batch_agg_kernel<4, 4, Spec12>;
+    case 13: return gb_batch_agg_kernel<4, 2, Spec13>;
+    case 14: return gb_batch_agg_kernel<4, 3, Spec14>;
+    case 15: return gb_batch_agg_kernel<4, 3, Spec15>;
     default: return max_st <= 4 ? gb_batch_agg_kernel<4, 4, SpecGeneric> : gb_batch_agg_kernel<2, 8, SpecGeneric>;
     }
 }
@@ -1013,7 +1029,15 @@ AggKernel staged_kernel_for(int spec) {
     case 4: return gb_staged_kernel<Spec4>;
     case 5: return gb_staged_kernel<Spec5>;
     case 6: return gb_staged_kernel<Spec6>;
-    default: return gb_staged_kernel<Spec7>;
+    case 7: return gb_staged_kernel<Spec7>;
+    case 8: return gb_staged_kernel<Spec8>;
+    case 9: return gb_staged_kernel<Spec9>;
+    case 10: return gb_staged_kernel<Spec10>;
+    case 11: return gb_staged_kernel<Spec11>;
+    case 12: return gb_staged_kernel<Spec12>;
+    case 13: return gb_staged_kernel<Spec13>;
+    case 14: return gb_staged_kernel<Spec14>;
+    default: return gb_staged_kernel<Spec15>;
     }
 }
 
@@ -1041,6 +1065,14 @@ int gb_spec_of(const StateDesc* st, int n) {
     if (spec_matches<Spec5>(st, n)) return 5;
     if (spec_matches<Spec6>(st, n)) return 6;
     if (spec_matches<Spec7>(st, n)) return 7;
+    if (spec_matches<Spec8>(st, n)) return 8;
+    if (spec_matches<Spec9>(st, n)) return 9;
+    if (spec_matches<Spec10>(st, n)) return 10;
+    if (spec_matches<Spec11>(st, n)) return 11;
+    if (spec_matches<Spec12>(st, n)) return 12;
+    if (spec_matches<Spec13>(st, n)) return 13;
+    if (spec_matches<Spec14>(st, n)) return 14;
+    if (spec_matches<Spec15>(st, n)) return 15;
     return 0;
 }
 
@@ -1542,13 +1574,13 @@ constexpr uint64_t BATCH_ALONE_ROWS = 1ull << 21;
 // one persistent launch per group.
 static bolt_status gb_run_aggregate(bolt_ctx* ctx, GbPlan** pls, int nq, cudaStream_t s, uint32_t flags) {
     if (nq == 1) return gb_agg_one(ctx, pls[0], s, flags);
-    std::vector<GbPlan*> groups[8];
+    std::vector<GbPlan*> groups[GB_SPECS + 1];
     for (int q = 0; q < nq; ++q) {
         if (pls[q]->prm.n_rows >= BATCH_ALONE_ROWS) {
             bolt_status st = gb_agg_one(ctx, pls[q], s, flags);
             if (st != BOLT_OK) return st;
         } else {
-            groups[std::min(std::max(pls[q]->prm.spec, 0), 7)].push_back(pls[q]);
+            groups[pls[q]->prm.spec].push_back(pls[q]);
         }
     }
     for (auto& g : groups) {

@@ -281,12 +281,22 @@ __device__ __forceinline__ void lean_rows(const GbParams& p, const GbPart& q, ul
                                           uint32_t* filt, uint32_t* s_nspill, uint32_t* s_stop, const TileCols& t,
                                           uint32_t first, int nchunks, uint32_t limit, uint16_t* list, LeanWarp& lw) {
     const uint32_t lane = lane_id();
-    uint32_t cnt = 0;
     const int32_t* pc = reinterpret_cast<const int32_t*>(t.pc);
+    if (!pc) {  // no WHERE: every row survives, in place
+        for (int c = 0; c < nchunks; ++c) {
+            const uint32_t i = first + (uint32_t)c * 32u + lane;
+            ull stored = 0, fw[GB_PART_MAX_FIELDS];
+            const bool in = i < limit;
+            if (in) load_row<KP>(q, t, i, stored, fw);
+            fold_step<SP, MISS>(p, q, sk, sw, fill, filt, s_nspill, s_stop, in, stored, fw, lw);
+        }
+        return;
+    }
+    uint32_t cnt = 0;
     for (int c = 0; c < nchunks; ++c) {
         const uint32_t i = first + (uint32_t)c * 32u + lane;
         bool ok = i < limit;
-        if (pc && ok) {
+        if (ok) {
             const int32_t v = pc[i];
             ok = ((v >= q.pred_lo) & (v <= q.pred_hi)) != (q.pred_neg != 0);
         }
@@ -800,8 +810,21 @@ LeanKernel lean_for_spec(int spec) {
     case 5: return gb_lean_kernel<KP, Spec5, MISS>;
     case 6: return gb_lean_kernel<KP, Spec6, MISS>;
     case 7: return gb_lean_kernel<KP, Spec7, MISS>;
-    default: return nullptr;
+    default: break;
     }
+    // Layouts the partitioned tier does not compile.
+    if constexpr (MISS == MISS_GLOBAL) {
+        switch (spec) {
+        case 8: return gb_lean_kernel<KP, Spec8, MISS>;
+        case 9: return gb_lean_kernel<KP, Spec9, MISS>;
+        case 10: return gb_lean_kernel<KP, Spec10, MISS>;
+        case 11: return gb_lean_kernel<KP, Spec11, MISS>;
+        case 12: return gb_lean_kernel<KP, Spec12, MISS>;
+        case 13: return gb_lean_kernel<KP, Spec13, MISS>;
+        default: break;
+        }
+    }
+    return nullptr;
 }
 
 template <int MISS>
