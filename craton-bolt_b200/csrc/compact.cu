@@ -894,15 +894,11 @@ bolt_status compact_common(bolt_ctx* ctx, const bolt_col_view* cols, int32_t n_c
     sp.n_out_dev = cnt;
     st = compact_enqueue(ctx, s, sp, flags);
     if (st != BOLT_OK) return st;
-    st = call_end(ctx, flags, s);
-    if (st != BOLT_OK) return st;
-    if (flags & BOLT_FLAG_ASYNC) return BOLT_OK;
+    if (flags & BOLT_FLAG_ASYNC) return call_end(ctx, flags, s);
     uint32_t f = 0;
-    st = read_status(ctx, s, 0, &f);
+    st = call_finish(ctx, flags, s, cnt, 1, &f);
     if (st != BOLT_OK) return st;
-    ull v = 0;
-    BOLT_CUDA(ctx, cudaMemcpy(&v, cnt, 8, cudaMemcpyDeviceToHost));
-    *n_out = v;
+    *n_out = ctx->h_words[2];
     return flags_to_status(ctx, f, "compaction");
 }
 

@@ -88,6 +88,22 @@ bolt_status call_end(bolt_ctx* ctx, uint32_t flags, cudaStream_t s) {
     return BOLT_OK;
 }
 
+bolt_status call_finish(bolt_ctx* ctx, uint32_t call_flags, cudaStream_t s, const ull* words, int n_words, uint32_t* flags) {
+    BOLT_CUDA(ctx, cudaGetLastError());
+    if (call_flags & BOLT_FLAG_PROFILE) BOLT_CUDA(ctx, cudaEventRecord(ctx->ev1, s));
+    BOLT_CUDA(ctx, cudaMemcpyAsync(ctx->h_words, ctx->d_status, 16, cudaMemcpyDeviceToHost, s));
+    if (n_words > 0)
+        BOLT_CUDA(ctx, cudaMemcpyAsync(ctx->h_words + 2, words, n_words * sizeof(ull), cudaMemcpyDeviceToHost, s));
+    BOLT_CUDA(ctx, cudaStreamSynchronize(s));
+    if (call_flags & BOLT_FLAG_PROFILE) {
+        float ms = 0.f;
+        BOLT_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
+        ctx->last_ms = ms;
+    }
+    *flags = (uint32_t)(ctx->h_words[0] & 0xFFFFFFFFu);
+    return BOLT_OK;
+}
+
 cudaError_t ensure_smem_optin(const void* kernel, int device, int max_optin) {
     static std::mutex mu;
     static std::set<std::pair<const void*, int>> done;

@@ -114,6 +114,11 @@ inline void kernel_mark_end(bolt_ctx* ctx, uint32_t flags, cudaStream_t s) {
     }
 }
 
+// call_end of a synchronous call together with its results: one wait for the
+// stream covers the profiling event, the status word (*flags) and `n_words`
+// device words, which land at ctx->h_words + 2.
+bolt_status call_finish(bolt_ctx* ctx, uint32_t call_flags, cudaStream_t s, const ull* words, int n_words, uint32_t* flags);
+
 // Reads the status word + n device words into ctx->h_words (synchronises s).
 bolt_status read_status(bolt_ctx* ctx, cudaStream_t s, int n_words, uint32_t* flags);
 

@@ -1805,14 +1805,12 @@ static bolt_status gb_single(bolt_ctx* ctx, const bolt_groupby_desc* d, bolt_gro
                 continue;
             }
             if (st != BOLT_OK) return st;
-            st = call_end(ctx, flags, s);
-            if (st != BOLT_OK) return st;
-            if (flags & BOLT_FLAG_ASYNC) return BOLT_OK;
+            if (flags & BOLT_FLAG_ASYNC) return call_end(ctx, flags, s);
             uint32_t f = 0;
-            st = read_status(ctx, s, 0, &f);
+            st = call_finish(ctx, flags, s, pl.words, 5, &f);
             if (st != BOLT_OK) return st;
-            ull w[5] = {0, 0, 0, 0, 0};
-            BOLT_CUDA(ctx, cudaMemcpy(w, pl.words, sizeof w, cudaMemcpyDeviceToHost));
+            ull w[5];
+            std::memcpy(w, ctx->h_words + 2, sizeof w);
             out->n_groups = w[2];
             const uint32_t bits = (uint32_t)w[4];
             if (f == 0 && pl.prm.i64_bits && bits + (uint32_t)ceil_log2_u64(pl.prm.n_rows + 1) >= 63) {
@@ -1857,14 +1855,12 @@ static bolt_status gb_single(bolt_ctx* ctx, const bolt_groupby_desc* d, bolt_gro
         GbPlan* one = &pl;
         st = gb_run(ctx, &one, 1, s, flags);
         if (st != BOLT_OK) return st;
-        st = call_end(ctx, flags, s);
-        if (st != BOLT_OK) return st;
-        if (flags & BOLT_FLAG_ASYNC) return BOLT_OK;
+        if (flags & BOLT_FLAG_ASYNC) return call_end(ctx, flags, s);
         uint32_t f = 0;
-        st = read_status(ctx, s, 0, &f);
+        st = call_finish(ctx, flags, s, pl.words, 5, &f);
         if (st != BOLT_OK) return st;
-        ull w[5] = {0, 0, 0, 0, 0};
-        BOLT_CUDA(ctx, cudaMemcpy(w, pl.words, sizeof w, cudaMemcpyDeviceToHost));
+        ull w[5];
+        std::memcpy(w, ctx->h_words + 2, sizeof w);
         out->n_groups = w[2];
         const uint32_t bits = (uint32_t)w[4];
         if (f == 0 && pl.prm.i64_bits && bits + (uint32_t)ceil_log2_u64(pl.prm.n_rows + 1) >= 63)

@@ -346,7 +346,8 @@ extern "C" bolt_status bolt_hash_join_build(bolt_ctx* ctx, const bolt_col_view* 
         payload ? (const int32_t*)payload->data : nullptr, n, ctx->d_status);
     kernel_mark_end(ctx, flags, s);
     ctx->last_launches = 1;
-    st = call_end(ctx, flags, s);
+    uint32_t f = 0;
+    st = flags & BOLT_FLAG_ASYNC ? call_end(ctx, flags, s) : call_finish(ctx, flags, s, nullptr, 0, &f);
     if (st != BOLT_OK) return st;
     bolt_join_table* t = new bolt_join_table();
     t->slots = slots;
@@ -357,9 +358,7 @@ extern "C" bolt_status bolt_hash_join_build(bolt_ctx* ctx, const bolt_col_view* 
     t->pinned_mark = 0;
     t->owner = ctx;
     if (!(flags & BOLT_FLAG_ASYNC)) {
-        uint32_t f = 0;
-        st = read_status(ctx, s, 0, &f);
-        if (st == BOLT_OK && f == ST_FLAG_DUPKEY) {
+        if (f == ST_FLAG_DUPKEY) {
             // Duplicate build keys: rebuild as a multi-match table.
             st = join_build_multi(ctx, s, t, build_key);
             if (st == BOLT_OK) st = read_status(ctx, s, 0, &f);
@@ -425,14 +424,10 @@ extern "C" bolt_status bolt_hash_join_probe(bolt_ctx* ctx, const bolt_join_table
         kernel_mark_end(ctx, flags, s);
         ctx->last_launches = 1;
     }
-    st = call_end(ctx, flags, s);
-    if (st != BOLT_OK) return st;
-    if (flags & BOLT_FLAG_ASYNC) return BOLT_OK;
+    if (flags & BOLT_FLAG_ASYNC) return call_end(ctx, flags, s);
     uint32_t f = 0;
-    st = read_status(ctx, s, 0, &f);
+    st = call_finish(ctx, flags, s, a.n_out, 1, &f);
     if (st != BOLT_OK) return st;
-    ull v = 0;
-    BOLT_CUDA(ctx, cudaMemcpy(&v, a.n_out, 8, cudaMemcpyDeviceToHost));
-    *n_out = v;
+    *n_out = ctx->h_words[2];
     return flags_to_status(ctx, f, "hash join probe");
 }

@@ -1387,11 +1387,9 @@ extern "C" bolt_status bolt_radix_sort_perm_multi(bolt_ctx* ctx, const bolt_col_
         cur = dst;
     }
     kernel_mark_end(ctx, flags, s);
-    st = call_end(ctx, flags, s);
-    if (st != BOLT_OK) return st;
-    if (flags & BOLT_FLAG_ASYNC) return BOLT_OK;
+    if (flags & BOLT_FLAG_ASYNC) return call_end(ctx, flags, s);
     uint32_t f = 0;
-    st = read_status(ctx, s, 0, &f);
+    st = call_finish(ctx, flags, s, nullptr, 0, &f);
     if (st != BOLT_OK) return st;
     return flags_to_status(ctx, f, "ORDER BY");
 }
