@@ -554,9 +554,10 @@ constexpr int FIN_CHUNK = 4096;
 constexpr int GATHER_CHUNK = 1024;
 
 // Occupied-slot compaction of the large-table queries: work items are
-// (query, chunk of 4096 slots); order key = packed key ^ sign bit.
+// (query, chunk of 4096 slots); order key = packed key ^ sign bit. One query
+// alone (fins null) passes its descriptor by value: no upload to wait for.
 __global__ void __launch_bounds__(256) gb_compact_batch_kernel(const GbFinal* fins, const uint32_t* begins, int nq,
-                                                                uint32_t total_items) {
+                                                                uint32_t total_items, const __grid_constant__ GbFinal one) {
     // Each warp takes runs of 32 x CMP_ROUNDS slots: it reads their keys,
     // counts the occupied ones with ballots, claims that many output rows
     // with one atomic, then writes them (one atomic per 512 slots instead of
@@ -568,9 +569,9 @@ __global__ void __launch_bounds__(256) gb_compact_batch_kernel(const GbFinal* fi
     for (uint32_t item = blockIdx.x; item < total_items; item += gridDim.x) {
         const int q = query_of(begins, nq, item);
         __syncthreads();
-        load_final(f, fins + q);
+        load_final(f, fins ? fins + q : &one);
         const ull cap = 1ull << f.log2cap;
-        const uint64_t c0 = (uint64_t)(item - begins[q]) * FIN_CHUNK;
+        const uint64_t c0 = (uint64_t)(item - (fins ? begins[q] : 0u)) * FIN_CHUNK;
         const uint64_t c1 = c0 + FIN_CHUNK < cap + 1 ? c0 + FIN_CHUNK : cap + 1;
         for (uint64_t run = c0 + (uint64_t)warp * 32 * CMP_ROUNDS; run < c1;
              run += (uint64_t)nwarps * 32 * CMP_ROUNDS) {
@@ -616,17 +617,17 @@ __global__ void __launch_bounds__(256) gb_compact_batch_kernel(const GbFinal* fi
 // Output rows of the large-table queries: work items are (query, chunk of
 // GATHER_CHUNK output rows) up to cap + 1 rows; rows past the group count exit.
 __global__ void __launch_bounds__(256) gb_gather_batch_kernel(const GbFinal* fins, const uint32_t* begins, int nq,
-                                                               uint32_t total_items) {
+                                                               uint32_t total_items, const __grid_constant__ GbFinal one) {
     __shared__ __align__(16) GbFinal f;
     for (uint32_t item = blockIdx.x; item < total_items; item += gridDim.x) {
         const int q = query_of(begins, nq, item);
         __syncthreads();
-        load_final(f, fins + q);
+        load_final(f, fins ? fins + q : &one);
         const ull cap = 1ull << f.log2cap;
         const ull G = min(*f.n_nonnull, f.n_max);  // (a counter that ran past the table flagged GROW)
         const bool has_null = f.gtab[(cap + 1) * (ull)f.slot_words] != 0;
         const ull total = G + (has_null ? 1 : 0);
-        const uint64_t c0 = (uint64_t)(item - begins[q]) * GATHER_CHUNK;
+        const uint64_t c0 = (uint64_t)(item - (fins ? begins[q] : 0u)) * GATHER_CHUNK;
         if (c0 == 0 && threadIdx.x == 0) {
             *f.n_groups = total;
             if (f.n_groups_user) *f.n_groups_user = total;
@@ -1652,24 +1653,29 @@ static bolt_status gb_run_finalize(bolt_ctx* ctx, GbPlan** pls, int nq, cudaStre
         }
         cbeg[nl] = (uint32_t)citems;
         gbeg[nl] = (uint32_t)gitems;
-        GbFinal* d_f = (GbFinal*)arena_alloc(ctx, sizeof(GbFinal) * nl);
-        uint32_t* d_beg = (uint32_t*)arena_alloc(ctx, 4ull * (nl + 1));
-        uint32_t* d_gbeg = (uint32_t*)arena_alloc(ctx, 4ull * (nl + 1));
-        if (!d_f || !d_beg || !d_gbeg)
-            return fail(ctx, BOLT_ERR_CAPACITY, "GROUP BY: scratch arena too small for the finalize");
-        bolt_status st = stage_upload(ctx, s, d_f, large.data(), sizeof(GbFinal) * nl);
-        if (st == BOLT_OK) st = stage_upload(ctx, s, d_beg, cbeg.data(), 4ull * (nl + 1));
-        if (st == BOLT_OK) st = stage_upload(ctx, s, d_gbeg, gbeg.data(), 4ull * (nl + 1));
-        if (st != BOLT_OK) return st;
+        GbFinal* d_f = nullptr;
+        uint32_t *d_beg = nullptr, *d_gbeg = nullptr;
+        bolt_status st = BOLT_OK;
+        if (nl > 1) {
+            d_f = (GbFinal*)arena_alloc(ctx, sizeof(GbFinal) * nl);
+            d_beg = (uint32_t*)arena_alloc(ctx, 4ull * (nl + 1));
+            d_gbeg = (uint32_t*)arena_alloc(ctx, 4ull * (nl + 1));
+            if (!d_f || !d_beg || !d_gbeg)
+                return fail(ctx, BOLT_ERR_CAPACITY, "GROUP BY: scratch arena too small for the finalize");
+            st = stage_upload(ctx, s, d_f, large.data(), sizeof(GbFinal) * nl);
+            if (st == BOLT_OK) st = stage_upload(ctx, s, d_beg, cbeg.data(), 4ull * (nl + 1));
+            if (st == BOLT_OK) st = stage_upload(ctx, s, d_gbeg, gbeg.data(), 4ull * (nl + 1));
+            if (st != BOLT_OK) return st;
+        }
         const unsigned cg = (unsigned)std::min<uint64_t>(citems, (uint64_t)ctx->num_sms * 8);
         if (!pls[large_q[0]]->precompacted) {  // (a precompacted query is finalized alone)
-            gb_compact_batch_kernel<<<cg, 256, 0, s>>>(d_f, d_beg, nl, (uint32_t)citems);
+            gb_compact_batch_kernel<<<cg, 256, 0, s>>>(d_f, d_beg, nl, (uint32_t)citems, large[0]);
             ctx->last_launches++;
         }
         st = radix_sort(ctx, s, sp);
         if (st != BOLT_OK) return st;
         const unsigned gg = (unsigned)std::min<uint64_t>(gitems, (uint64_t)ctx->num_sms * 8);
-        gb_gather_batch_kernel<<<gg, 256, 0, s>>>(d_f, d_gbeg, nl, (uint32_t)gitems);
+        gb_gather_batch_kernel<<<gg, 256, 0, s>>>(d_f, d_gbeg, nl, (uint32_t)gitems, large[0]);
         ctx->last_launches++;
     }
     BOLT_CUDA(ctx, cudaGetLastError());

@@ -30,9 +30,9 @@
 // 2^28 uniform 64-bit keys take two passes and the local step instead of
 // eight passes (19.2 -> 8.4 ms: histogram 1.0, two passes 4.6, local step
 // 2.7; 30M keys 2.29 -> 1.05 ms, 30M uniform 32-bit keys 0.93 -> 0.83 ms).
-// Segments with few varying digits, or whose keys crowd into long runs (a
-// value shared by 1 % of 2^28 rows: 19.2 -> 19.4 ms), keep the full LSD
-// schedule.
+// A value shared by many rows is let through in a sweep (1 % of 2^28 rows:
+// 19.1 -> 10.3 ms). Segments with few varying digits, or whose keys crowd
+// into long runs of many values, keep the full LSD schedule.
 #include "radix_sort.cuh"
 
 #include "bulk.cuh"
@@ -97,6 +97,12 @@ struct SegDesc {
     uint32_t loc_begin;
 };
 
+// A run of equal top digits longer than a window: rows [s, e) of segment sg.
+struct LongRun {
+    ull s, e;
+    ull sg;
+};
+
 // What sort_plan_kernel decided for one segment.
 struct SegPlan {
     uint32_t sched;  // digits that get a pass (bit p)
@@ -109,8 +115,9 @@ struct SortArgs {
     int32_t desc;
     int32_t indirect;
     int32_t nseg;
-    const SegDesc* segs;
-    const uint32_t* item_begins;  // nseg + 1
+    const SegDesc* segs;          // nullptr for one segment: seg0 (no descriptor upload before the first launch)
+    SegDesc seg0;
+    const uint32_t* item_begins;  // nseg + 1; the three begins are not read for one segment
     const uint32_t* hist_begins;  // nseg + 1
     const uint32_t* loc_begins;   // nseg + 1
     void* kA;
@@ -126,7 +133,8 @@ struct SortArgs {
     uint32_t total_hist_items;
     uint32_t total_loc_items;
     uint32_t loc_range;    // rows of one work item of the local step
-    uint32_t* tile_ctr;    // NPASS + 1 (the last: the local step's items)
+    uint32_t* tile_ctr;    // NPASS + 2 (the last two: the local step's items, long runs found)
+    LongRun* longs;
     uint32_t* status;
 };
 
@@ -186,6 +194,8 @@ __device__ __forceinline__ int seg_of(const uint32_t* begins, int nseg, uint32_t
     return lo;
 }
 
+__device__ __forceinline__ const SegDesc& seg_desc(const SortArgs& a, int sg) { return a.segs ? a.segs[sg] : a.seg0; }
+
 // Rows of a segment: the device count when given, never more than the
 // segment's buffers hold (a producer that ran out of room may count past it).
 __device__ __forceinline__ uint64_t seg_n(const SegDesc& d) {
@@ -199,14 +209,14 @@ __device__ __forceinline__ uint64_t seg_n(const SegDesc& d) {
 // every counter in neighbouring banks changed nothing). A CTA flushes its
 // counters once per segment it meets.
 template <typename K>
-__global__ void __launch_bounds__(HIST_BLOCK) sort_hist_kernel(SortArgs a) {
+__global__ void __launch_bounds__(HIST_BLOCK) sort_hist_kernel(const __grid_constant__ SortArgs a) {
     constexpr int NP = KeyTraits<K>::NPASS;
     __shared__ uint32_t h[NP * 256];
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     // Clear the first look-back buffer and the pass tile counters.
     for (uint64_t i = tid; i < a.lb_stride; i += stride) a.lookback[i] = 0;
-    if (blockIdx.x == 0 && threadIdx.x < NP + 1) a.tile_ctr[threadIdx.x] = 0;
+    if (blockIdx.x == 0 && threadIdx.x < NP + 2) a.tile_ctr[threadIdx.x] = 0;
     for (int i = threadIdx.x; i < NP * 256; i += blockDim.x) h[i] = 0;
     int cur = -1;
     auto flush = [&]() {
@@ -225,7 +235,7 @@ __global__ void __launch_bounds__(HIST_BLOCK) sort_hist_kernel(SortArgs a) {
             __syncthreads();
             cur = sg;
         }
-        const SegDesc& d = a.segs[sg];
+        const SegDesc& d = seg_desc(a, sg);
         const uint64_t n = seg_n(d);
         const uint64_t c0 = (uint64_t)(item - d.hist_begin) * HIST_CHUNK;
         const uint64_t c1 = c0 + HIST_CHUNK < n ? c0 + HIST_CHUNK : n;
@@ -302,64 +312,85 @@ __device__ __forceinline__ void block_min_max(K& mn, K& mx, ull* red) {
 // histogram says it, for more it is estimated from the agreeing pairs of a
 // sample, counted in a shared hash table (2^28 uniform keys, k = 2: 512 pairs
 // of 8,192 samples expected for the true 4,096); a single long run that the
-// mean does not show is seen as many samples in one run. All of it only
+// mean does not show is seen as many samples in one run. A run that is mostly
+// one value (zeros, infinities, a default) counts by its other samples only:
+// the local step lets the value's rows through in one sweep. All of it only
 // steers the speed: the local step orders runs of any length.
 struct SampleRuns {
     ull pairs;     // agreeing pairs
     ull longest;   // most samples in one run
+    ull hottest;   // most samples of one value left out of the two
 };
 
 // Counts the runs of equal key >> sh among the block's samples (cnt_s per
-// thread). tab: 32-bit hashes of the prefixes, mask + 1 slots, half empty.
+// thread). tab: 32-bit hashes of the prefixes, mask + 1 slots, half empty;
+// cnt: samples | samples that differ from the slot's first << 16; fst: hash
+// of the slot's first key.
 template <typename K>
 __device__ __forceinline__ SampleRuns sample_runs(const K (&smp)[PLAN_PER], int cnt_s, int sh, uint32_t mask, uint32_t* tab,
-                                                  uint32_t* cnt, ull* red) {
+                                                  uint32_t* cnt, uint32_t* fst, ull* red) {
     __syncthreads();
     for (uint32_t i = threadIdx.x; i <= mask; i += PLAN_BLOCK) {
         tab[i] = 0;
         cnt[i] = 0;
+        fst[i] = 0;
     }
     __syncthreads();
-    ull pairs = 0;
-    uint32_t longest = 0;
 #pragma unroll
     for (int u = 0; u < PLAN_PER; ++u) {
         if (u >= cnt_s) continue;
         const ull hp = (ull)(smp[u] >> sh) * 0x9E3779B97F4A7C15ull;
         const uint32_t sig = (uint32_t)(hp >> 32) | 1u;
+        const uint32_t own = (uint32_t)(((ull)smp[u] * 0xD6E8FEB86659FD93ull) >> 32) | 1u;
         uint32_t h = (uint32_t)(hp >> 40) & mask;
         for (uint32_t probe = 0; probe <= mask; ++probe) {
             const uint32_t old = atomicCAS(&tab[h], 0u, sig);
             if (old == 0 || old == sig) {
-                const uint32_t c = atomicAdd(&cnt[h], 1u);
-                pairs += c;
-                longest = max(longest, c + 1);
+                const uint32_t f = atomicCAS(&fst[h], 0u, own);
+                atomicAdd(&cnt[h], f == 0 || f == own ? 1u : 0x10001u);
                 break;
             }
             h = (h + 1) & mask;
         }
     }
+    __syncthreads();
+    ull pairs = 0;
+    uint32_t longest = 0, hottest = 0;
+    for (uint32_t i = threadIdx.x; i <= mask; i += PLAN_BLOCK) {
+        const uint32_t all = cnt[i] & 0xFFFFu, other = cnt[i] >> 16, same = all - other;
+        uint32_t c = all;
+        if (same >= 4 && other * 4 <= all) {
+            c = other + 1;
+            hottest = max(hottest, same);
+        }
+        pairs += (ull)c * (c ? c - 1 : 0) / 2;
+        longest = max(longest, c);
+    }
     SampleRuns r;
     r.pairs = block_sum(pairs, red);
     longest = __reduce_max_sync(0xffffffffu, longest);
+    hottest = __reduce_max_sync(0xffffffffu, hottest);
     __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = longest;
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = (ull)longest << 32 | hottest;
     __syncthreads();
-    r.longest = __reduce_max_sync(0xffffffffu, (uint32_t)red[threadIdx.x & 31]);
+    const ull m = red[threadIdx.x & 31];
+    r.longest = __reduce_max_sync(0xffffffffu, (uint32_t)(m >> 32));
+    r.hottest = __reduce_max_sync(0xffffffffu, (uint32_t)m);
     return r;
 }
 
 template <typename K>
-__global__ void __launch_bounds__(PLAN_BLOCK) sort_plan_kernel(SortArgs a) {
+__global__ void __launch_bounds__(PLAN_BLOCK) sort_plan_kernel(const __grid_constant__ SortArgs a) {
     constexpr int NP = KeyTraits<K>::NPASS;
     constexpr uint32_t CAP = LOC_BLOCK * KeyTraits<K>::LOC_ITEMS;
     extern __shared__ __align__(16) unsigned char plan_sm[];
     uint32_t* tab = reinterpret_cast<uint32_t*>(plan_sm);  // 2 * PLAN_SAMPLES words
     uint32_t* cnt = tab + 2 * PLAN_SAMPLES;                // 2 * PLAN_SAMPLES words
+    uint32_t* fst = cnt + 2 * PLAN_SAMPLES;                // 2 * PLAN_SAMPLES words
     __shared__ uint32_t s_act;
     __shared__ ull red[PLAN_BLOCK / 32];
     const int sg = blockIdx.x;
-    const SegDesc& d = a.segs[sg];
+    const SegDesc& d = seg_desc(a, sg);
     const uint64_t n = seg_n(d);
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     if (t == 0) s_act = 0;
@@ -424,9 +455,10 @@ __global__ void __launch_bounds__(PLAN_BLOCK) sort_plan_kernel(SortArgs a) {
                 mean = (double)block_sum((ull)c * c, red) / (double)n;
                 many = __syncthreads_or(c > CAP + n / 2048);
             } else {
-                const SampleRuns runs = sample_runs<K>(smp, cnt_s, 8 * top, 2 * m - 1, tab, cnt, red);
+                const SampleRuns runs = sample_runs<K>(smp, cnt_s, 8 * top, 2 * m - 1, tab, cnt, fst, red);
                 mean = rows_per_pair * (double)runs.pairs;
-                many = runs.longest >= 6 && runs.longest * step > CAP + n / 2048;
+                // (one CTA sweeps a hot value's run: 1/64 of the rows at most)
+                many = (runs.longest >= 6 && runs.longest * step > CAP + n / 2048) || runs.hottest * step > n / 64;
             }
             if (!many && mean <= KeyTraits<K>::LOC_FULL * CAP) {
                 plan = {sched, 1u, act};
@@ -438,7 +470,7 @@ __global__ void __launch_bounds__(PLAN_BLOCK) sort_plan_kernel(SortArgs a) {
 }
 
 template <typename K>
-__global__ void __launch_bounds__(SORT_BLOCK, 3) sort_pass_kernel(SortArgs a, int p) {
+__global__ void __launch_bounds__(SORT_BLOCK, 3) sort_pass_kernel(const __grid_constant__ SortArgs a, int p) {
     constexpr int NW = SORT_BLOCK / 32;
     constexpr int SORT_ITEMS = KeyTraits<K>::ITEMS;
     constexpr int SORT_TILE = KeyTraits<K>::TILE;
@@ -469,7 +501,7 @@ __global__ void __launch_bounds__(SORT_BLOCK, 3) sort_pass_kernel(SortArgs a, in
         const uint32_t item = s_item;
         if (item >= a.total_items) return;
         const int sg = seg_of(a.item_begins, a.nseg, item);
-        const SegDesc& d = a.segs[sg];
+        const SegDesc& d = seg_desc(a, sg);
         const SegPlan plan = a.plan[sg];
         const uint32_t active = plan.sched;
         if (!((active >> p) & 1u)) continue;
@@ -714,11 +746,11 @@ __device__ __forceinline__ uint64_t run_start_from(const K* keys, uint64_t p, ui
 // Stable LSD radix sort of the rows [s, e) by one CTA, tile after tile, over
 // the digits that vary among them; the sorted payloads go to `out`. For the
 // rare runs longer than a window. It orders row numbers, in the
-// other ping-pong buffer's memory, and leaves the rows where they are: the
-// neighbouring work item may be searching them for its first run. src_in_a:
-// which buffer holds the rows; cnt: LOC_NW * 256 words; base: 256 words.
+// other ping-pong buffer's memory, and leaves the rows where they are.
+// src_in_a: which buffer holds the rows; cnt: LOC_NW * 256 words; base: 256
+// words.
 template <typename K>
-__device__ __noinline__ void local_serial_sort(K* kA, K* kB, uint32_t* pA, uint32_t* pB, bool src_in_a, uint64_t s,
+__device__ __forceinline__ void local_serial_sort(K* kA, K* kB, uint32_t* pA, uint32_t* pB, bool src_in_a, uint64_t s,
                                                uint64_t e, uint32_t* out, uint32_t* cnt, uint32_t* base, ull* red) {
     constexpr int NP = KeyTraits<K>::NPASS;
     const int t = threadIdx.x, w = t >> 5, lane = t & 31;
@@ -904,8 +936,8 @@ __device__ __forceinline__ void local_pass(const uint16_t* src, uint16_t* dst, b
 // the keys in order, all varying digits are sorted.
 template <typename K>
 __device__ __noinline__ void local_radix_sort(const K* skey, const uint32_t* spay, uint16_t* ia, uint16_t* ib, uint32_t len,
-                                              uint32_t act, K lo, int bits, uint32_t* out, uint32_t* cnt, uint32_t* wsum,
-                                              ull* red) {
+                                              uint32_t act, K lo, int bits, uint32_t* out, uint32_t gap_at, uint64_t gap,
+                                              uint32_t* cnt, uint32_t* wsum, ull* red) {
     constexpr int ITEMS = KeyTraits<K>::LOC_ITEMS;
     const int t = threadIdx.x;
     const Packer pack(act, (int)sizeof(K));
@@ -938,8 +970,118 @@ __device__ __noinline__ void local_radix_sort(const K* skey, const uint32_t* spa
             cur = src;
         }
     }
-    for (uint32_t p = t; p < len; p += LOC_BLOCK) out[p] = spay[cur[p]];
+    for (uint32_t p = t; p < len; p += LOC_BLOCK) out[p + (p >= gap_at ? gap : 0)] = spay[cur[p]];
     __syncthreads();
+}
+
+// A run [s, e) longer than a window in which one value is so frequent that
+// the rows of any other fit a window: a sweep counts the rows below and equal
+// to it, a second one writes the equal rows' payloads in place and collects
+// the others, in order, at skey / spay, where local_radix_sort orders them
+// around the gap. False (nothing written) when no value is that frequent.
+template <typename K>
+__device__ __forceinline__ bool local_hot_run(const K* kin, const uint32_t* pin, uint64_t s, uint64_t e, uint32_t cap, K* skey,
+                                           uint32_t* spay, uint16_t* ia, uint32_t act, K lo, int bits, uint32_t* out,
+                                           uint32_t* cnt, uint32_t* wsum, ull* red) {
+    constexpr int U = 8;
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+    const uint64_t len = e - s;
+    // Candidate: the most frequent of 32 samples (every warp finds the same).
+    const K mine = kin[s + (len / 32) * (uint32_t)lane + len / 64];
+    const uint32_t same = (uint32_t)__popc(__match_any_sync(0xffffffffu, mine));
+    const uint32_t best = __reduce_max_sync(0xffffffffu, same);
+    if (best < 8) return false;
+    const K hot = __shfl_sync(0xffffffffu, mine, __ffs(__ballot_sync(0xffffffffu, same == best)) - 1);
+    ull below = 0, equal = 0;
+    for (uint64_t i0 = t; i0 < len; i0 += LOC_BLOCK * U) {
+        K k[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint64_t i = i0 + (uint64_t)u * LOC_BLOCK;
+            k[u] = i < len ? kin[s + i] : ~(K)0;
+            if (i < len) {
+                below += k[u] < hot;
+                equal += k[u] == hot;
+            }
+        }
+    }
+    below = block_sum(below, red);
+    equal = block_sum(equal, red);
+    if (len - equal > cap) return false;
+    uint64_t rest = 0;  // rows of other values before the tile
+    for (uint64_t t0 = 0; t0 < len; t0 += LOC_BLOCK * U) {
+        // Warp w's part: rows t0 + w * 32 * U + [0, 32 * U), 32 at a time.
+        K k[U];
+        uint32_t pay[U], me[U], c = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint64_t i = t0 + (uint64_t)(w * U + u) * 32 + lane;
+            k[u] = i < len ? kin[s + i] : hot;
+            pay[u] = i < len ? pin[s + i] : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            me[u] = __ballot_sync(0xffffffffu, k[u] != hot);
+            c += __popc(me[u]);
+        }
+        __syncthreads();
+        if (lane == 0) wsum[w] = c;
+        __syncthreads();
+        const uint32_t v = lane < LOC_NW ? wsum[lane] : 0u;
+        uint32_t before = __reduce_add_sync(0xffffffffu, lane < w ? v : 0u);  // others in the earlier warps' parts
+        const uint32_t all = __reduce_add_sync(0xffffffffu, v);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint64_t i = t0 + (uint64_t)(w * U + u) * 32 + lane;
+            if (i < len) {
+                const uint64_t others = rest + before + __popc(me[u] & lanemask_lt());
+                if ((me[u] >> lane) & 1u) {
+                    skey[others] = k[u];
+                    spay[others] = pay[u];
+                } else {
+                    out[s + below + (i - others)] = pay[u];
+                }
+            }
+            before += __popc(me[u]);
+        }
+        rest += all;
+    }
+    __syncthreads();
+    local_radix_sort<K>(skey, spay, ia, ia + cap, (uint32_t)(len - equal), act, lo, bits, out + s, (uint32_t)below, equal, cnt,
+                        wsum, red);
+    return true;
+}
+
+// The runs longer than a window, one CTA each.
+template <typename K>
+__global__ void __launch_bounds__(LOC_BLOCK) sort_long_kernel(const __grid_constant__ SortArgs a) {
+    constexpr uint32_t CAP = LOC_BLOCK * KeyTraits<K>::LOC_ITEMS;
+    extern __shared__ __align__(16) unsigned char loc_sm[];
+    __shared__ uint32_t s_base[256], s_wsum[LOC_NW];
+    __shared__ ull red[2 * LOC_NW];
+    K* skey = reinterpret_cast<K*>(loc_sm);
+    uint32_t* bins = reinterpret_cast<uint32_t*>(skey + CAP);
+    uint32_t* spay = bins + LOC_WORDS;
+    uint16_t* ia = reinterpret_cast<uint16_t*>(spay + CAP);
+    const uint32_t runs = a.tile_ctr[KeyTraits<K>::NPASS + 1];
+    for (uint32_t r = blockIdx.x; r < runs; r += gridDim.x) {
+        const LongRun run = a.longs[r];
+        const SegDesc& d = seg_desc(a, (int)run.sg);
+        const SegPlan plan = a.plan[run.sg];
+        K* kA = (K*)a.kA + d.buf_off;
+        K* kB = (K*)a.kB + d.buf_off;
+        uint32_t* pA = a.pA + d.buf_off;
+        uint32_t* pB = a.pB + d.buf_off;
+        const bool in_a = (__popc(plan.sched) & 1) != 0;
+        const K* kin = in_a ? kA : kB;
+        const Packer pack(plan.act, (int)sizeof(K));
+        const int psh = 8 * (__popc(plan.act) - __popc(plan.sched));
+        const K lo = (K)((pack(kin[run.s]) >> psh) << psh);
+        if (!local_hot_run<K>(kin, in_a ? pA : pB, run.s, run.e, CAP, skey, spay, ia, plan.act, lo, psh, d.payload_out, bins,
+                              s_wsum, red))
+            local_serial_sort<K>(kA, kB, pA, pB, in_a, run.s, run.e, d.payload_out, bins, s_base, red);
+        __syncthreads();
+    }
 }
 
 // The local step: rows sorted by their top digits (key >> sh, the "prefix")
@@ -955,7 +1097,7 @@ __device__ __noinline__ void local_radix_sort(const K* skey, const uint32_t* spa
 // counter add, one staged key, a compare or two, one staged payload; reads
 // 12 B and writes 4 B per row.
 template <typename K>
-__global__ void __launch_bounds__(LOC_BLOCK, 2) sort_local_kernel(SortArgs a) {
+__global__ void __launch_bounds__(LOC_BLOCK, 2) sort_local_kernel(const __grid_constant__ SortArgs a) {
     constexpr int ITEMS = KeyTraits<K>::LOC_ITEMS;
     constexpr uint32_t CAP = LOC_BLOCK * ITEMS;
     extern __shared__ __align__(16) unsigned char loc_sm[];
@@ -964,7 +1106,7 @@ __global__ void __launch_bounds__(LOC_BLOCK, 2) sort_local_kernel(SortArgs a) {
     uint32_t* spay = bins + LOC_WORDS;                         // payloads in chunk order
     uint32_t* smeta = spay + CAP;                              // binned: position in the chunk, bin's length << 16, arrival << 24
     uint16_t* woff = reinterpret_cast<uint16_t*>(smeta + CAP);  // LOC_WORDS: keys before each word's bins
-    __shared__ uint32_t s_item, s_heavy, s_last, s_base[256];
+    __shared__ uint32_t s_item, s_heavy, s_last;
     __shared__ uint64_t s_lim[2];
     __shared__ uint32_t s_wsum[LOC_NW];
     __shared__ ull red[2 * LOC_NW];
@@ -977,7 +1119,7 @@ __global__ void __launch_bounds__(LOC_BLOCK, 2) sort_local_kernel(SortArgs a) {
         const uint32_t item = s_item;
         if (item >= a.total_loc_items) return;
         const int sg = seg_of(a.loc_begins, a.nseg, item);
-        const SegDesc& d = a.segs[sg];
+        const SegDesc& d = seg_desc(a, sg);
         const SegPlan plan = a.plan[sg];
         if (!plan.local) continue;
         const uint64_t n = seg_n(d);
@@ -1048,13 +1190,17 @@ __global__ void __launch_bounds__(LOC_BLOCK, 2) sort_local_kernel(SortArgs a) {
                 }
             }
             if (len == 0) {  // one run longer than the window
+                // (sort_long_kernel orders it: its code would cost this
+                // kernel's main path registers)
                 if (w == 0) {
                     const uint64_t at = run_start_from<K>(kin, pos + win, n, sh);
-                    if (lane == 0) s_lim[0] = at;
+                    if (lane == 0) {
+                        s_lim[0] = at;
+                        a.longs[atomicAdd(&a.tile_ctr[KeyTraits<K>::NPASS + 1], 1u)] = LongRun{pos, at, (ull)sg};
+                    }
                 }
                 __syncthreads();
                 const uint64_t e = s_lim[0];
-                local_serial_sort<K>(kA, kB, pA, pB, in_a, pos, e, d.payload_out, bins, s_base, red);
                 pos = e;
                 continue;
             }
@@ -1107,7 +1253,8 @@ __global__ void __launch_bounds__(LOC_BLOCK, 2) sort_local_kernel(SortArgs a) {
                 }
                 __syncthreads();
                 uint16_t* ia = reinterpret_cast<uint16_t*>(smeta);
-                local_radix_sort<K>(skey, spay, ia, ia + CAP, len, plan.act, lo, bits, d.payload_out + pos, bins, s_wsum, red);
+                local_radix_sort<K>(skey, spay, ia, ia + CAP, len, plan.act, lo, bits, d.payload_out + pos, len, 0, bins, s_wsum,
+                                    red);
                 pos += len;
                 continue;
             }
@@ -1231,8 +1378,9 @@ bolt_status run_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
     a.loc_range = (uint32_t)loc_range;
     a.lb_stride = items * 256;
     const uint64_t nb = end_n ? end_n : 1;
-    SegDesc* d_segs = (SegDesc*)arena_alloc(ctx, sizeof(SegDesc) * nseg);
-    uint32_t* d_begins = (uint32_t*)arena_alloc(ctx, 4 * begins.size());
+    const bool many = nseg > 1;
+    SegDesc* d_segs = many ? (SegDesc*)arena_alloc(ctx, sizeof(SegDesc) * nseg) : nullptr;
+    uint32_t* d_begins = many ? (uint32_t*)arena_alloc(ctx, 4 * begins.size()) : nullptr;
     a.kA = arena_alloc(ctx, nb * sizeof(K));
     a.kB = arena_alloc(ctx, nb * sizeof(K));
     a.pA = (uint32_t*)arena_alloc(ctx, nb * 4);
@@ -1242,23 +1390,28 @@ bolt_status run_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
     a.plan = (SegPlan*)arena_alloc(ctx, (uint64_t)nseg * sizeof(SegPlan));
     a.lookback = (uint32_t*)arena_alloc(ctx, 2 * a.lb_stride * 4);
     a.tile_ctr = (uint32_t*)arena_alloc(ctx, 64);
+    constexpr uint64_t LOC_CAP = (uint64_t)LOC_BLOCK * KeyTraits<K>::LOC_ITEMS;
+    a.longs = (LongRun*)arena_alloc(ctx, (sum_n / LOC_CAP + 1) * sizeof(LongRun));
     a.status = ctx->d_status;
-    if (!d_segs || !d_begins || !a.kA || !a.kB || !a.pA || !a.pB || !a.hist || !a.digit_base || !a.plan ||
+    if (!a.longs || (many && (!d_segs || !d_begins)) || !a.kA || !a.kB || !a.pA || !a.pB || !a.hist || !a.digit_base || !a.plan ||
         !a.lookback || !a.tile_ctr)
         return fail(ctx, BOLT_ERR_CAPACITY, "radix sort: scratch arena too small for %llu rows", (ull)total_n);
     a.segs = d_segs;
-    a.item_begins = d_begins;
-    a.hist_begins = d_begins + nseg + 1;
-    a.loc_begins = d_begins + 2 * (nseg + 1);
-    bolt_status st = stage_upload(ctx, s, d_segs, segs.data(), sizeof(SegDesc) * nseg);
-    if (st != BOLT_OK) return st;
-    st = stage_upload(ctx, s, d_begins, begins.data(), 4 * begins.size());
-    if (st != BOLT_OK) return st;
+    a.seg0 = segs[0];
+    if (many) {
+        a.item_begins = d_begins;
+        a.hist_begins = d_begins + nseg + 1;
+        a.loc_begins = d_begins + 2 * (nseg + 1);
+        bolt_status st = stage_upload(ctx, s, d_segs, segs.data(), sizeof(SegDesc) * nseg);
+        if (st != BOLT_OK) return st;
+        st = stage_upload(ctx, s, d_begins, begins.data(), 4 * begins.size());
+        if (st != BOLT_OK) return st;
+    }
     BOLT_CUDA(ctx, cudaMemsetAsync(a.hist, 0, (uint64_t)nseg * NP * 256 * 4, s));
     const unsigned hb = (unsigned)std::min<uint64_t>(hitems, (uint64_t)ctx->num_sms * 8);
     sort_hist_kernel<K><<<hb, HIST_BLOCK, 0, s>>>(a);
     BOLT_CUDA(ctx, smem_optin(sort_plan_kernel<K>, ctx));
-    sort_plan_kernel<K><<<nseg, PLAN_BLOCK, 2 * PLAN_SAMPLES * 8, s>>>(a);
+    sort_plan_kernel<K><<<nseg, PLAN_BLOCK, 2 * PLAN_SAMPLES * 12, s>>>(a);
     ctx->last_launches += 2;
     const size_t dyn = (sizeof(K) + 5) * SORT_TILE;
     BOLT_CUDA(ctx, smem_optin(sort_pass_kernel<K>, ctx));
@@ -1271,6 +1424,12 @@ bolt_status run_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
     const unsigned lg = (unsigned)std::min<uint64_t>(litems, (uint64_t)ctx->num_sms * 2);
     sort_local_kernel<K><<<lg, LOC_BLOCK, local_smem<K>(), s>>>(a);
     ctx->last_launches++;
+    if (sum_n > LOC_CAP) {
+        BOLT_CUDA(ctx, smem_optin(sort_long_kernel<K>, ctx));
+        const unsigned rg = (unsigned)std::min<uint64_t>(sum_n / LOC_CAP, (uint64_t)ctx->num_sms);
+        sort_long_kernel<K><<<rg, LOC_BLOCK, local_smem<K>(), s>>>(a);
+        ctx->last_launches++;
+    }
     BOLT_CUDA(ctx, cudaGetLastError());
     return BOLT_OK;
 }
@@ -1280,7 +1439,7 @@ bolt_status run_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
 uint64_t radix_sort_scratch(uint64_t total_n, uint64_t nseg, int32_t src) {
     const uint64_t ksz = (src == SRC_I32 || src == SRC_F32 || src == SRC_U32) ? 4 : 8;
     const uint64_t items = total_n / SORT_TILE_MIN + nseg + 1;
-    return 2 * total_n * (ksz + 4) + 2 * items * 256 * 4 + nseg * (2 * 8 * 256 * 4 + 512) + 64 * 1024;
+    return 2 * total_n * (ksz + 4) + total_n / 200 + 2 * items * 256 * 4 + nseg * (2 * 8 * 256 * 4 + 512) + 64 * 1024;
 }
 
 bolt_status radix_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {

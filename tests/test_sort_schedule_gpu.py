@@ -69,6 +69,26 @@ def test_i32_and_floats(bolt, engine, name, n):
         assert np.array_equal(got, np.argsort(f, kind="stable"))
 
 
+def test_runs_longer_than_a_window(bolt, engine):
+    """Runs of equal top digits past the local step's window, few enough rows to stay on the short schedule: of
+    many values, of one value among others of its run, and of one value alone."""
+    n = 3_000_017
+    v = _keys("full", n)
+    rng = np.random.default_rng(3)
+    at = rng.permutation(n)[: 9 * 8000].reshape(9, 8000)
+    for i in range(3):
+        v[at[i]] = (np.int64(0x1111111 * (i + 1)) << 32) | rng.integers(0, 1 << 32, 8000)
+        v[at[3 + i]] = np.int64(0x2222222222 * (i + 1))
+        v[at[6 + i]] = (np.int64(-0x3333333 * (i + 1)) << 32) | np.where(rng.random(8000) < 0.6, 77, rng.integers(0, 1 << 20, 8000))
+    got = engine.sort_indices([bolt.col(v).to("cuda")]).cpu().numpy().view(np.uint32)
+    assert np.array_equal(got, np.argsort(v, kind="stable"))
+    f = rng.normal(0, 1e3, n)
+    f[at[0]], f[at[1]], f[at[2]], f[at[3]] = 0.0, -0.0, np.nan, np.inf
+    for x in (f, f.astype(np.float32)):
+        got = engine.sort_indices([bolt.col(x).to("cuda")]).cpu().numpy().view(np.uint32)
+        assert np.array_equal(got, np.argsort(x, kind="stable"))
+
+
 @pytest.mark.parametrize("n", [4097, 250_007])
 def test_two_keys_with_nulls(bolt, engine, n):
     """Row ids as payload and NULL rows split off, through both schedules (the first key has few digits)."""
