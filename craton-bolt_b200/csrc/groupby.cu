@@ -240,6 +240,149 @@ __global__ void __launch_bounds__(512, SP::generic ? 1 : 2) gb_agg_kernel(const 
     gb_flush_shared(p, sk, sw, C);
 }
 
+// The fused join GROUP BY over dense columns (no validity): COUNT(*) and one
+// SUM per matched build payload. The random slot reads set its floor (a
+// 128-byte DRAM line per 16-byte slot of a table that outgrows L2), but the
+// general loop spent 450 instructions a row on dtype and validity switches,
+// 64-bit hashing and its rolled row loop, and waited for those instead. Here
+// the key width and the sum are compiled in, a step reads the home sectors of
+// U rows together with their values and the next step's keys, and a group is
+// found by a 32-bit hash of the payload (200M probes of 10M keys 4,970 ->
+// 4,500 us, then at 84 % of the copy rate; 40M probes of 1M keys 940 -> 580
+// us the whole call). Four rows a step were slower (5,280 us) than two.
+template <typename KT, class SP, int U>
+__global__ void __launch_bounds__(512, 2) gb_join_lean_kernel(const __grid_constant__ GbParams p) {
+    extern __shared__ __align__(16) ull smem[];
+    __shared__ uint32_t s_fill;
+    constexpr int KIND = SP::kind(1);
+    const int SW = p.sslot_words - 1;
+    const int C = 1 << p.smem_log2;
+    ull* sk = smem;
+    ull* sw = smem + C;
+    for (int i = threadIdx.x; i < C * (SW + 1); i += blockDim.x) smem[i] = 0;
+    if (threadIdx.x == 0) s_fill = 0;
+    __syncthreads();
+    const KT* keys = reinterpret_cast<const KT*>(p.jkey) + p.row_begin;
+    const uint32_t n = (uint32_t)p.n_rows;  // (below 2^31: the launch checks)
+    const uint32_t tile = blockDim.x * U, step = gridDim.x * tile;
+    uint32_t inserts = 0, pending = 0, absbits = 0, rounds = 0;
+    bool look = false;  // this lane's row found the global table full
+    const int w0 = p.st[0].sword - 1, w1 = p.st[1].sword - 1;
+    auto fold = [&](int32_t g, ull lo, bool fits) {
+        ull c1 = 0, c0 = lo;
+        if constexpr (KIND == K_SUM_D64 || KIND == K_SUM_I64) {
+            if (KIND == K_SUM_D64 && !fits) {
+                atomicOr(p.status, ST_FLAG_DECRANGE);
+                lo = 0;
+            }
+            if (KIND == K_SUM_I64) {
+                const ll v = (ll)lo;
+                const ull a = v < 0 ? (ull)(-(v + 1)) + 1ull : (ull)v;
+                absbits = max(absbits, 64u - (uint32_t)__clzll((ll)a));
+            }
+            c0 = lo & 0xFFFFFFFFull;
+            c1 = (ull)((ll)lo >> 32);
+        }
+        const ull stored = ~(ull)(ll)g;
+        if (stored == 0) {  // the group whose complement is 0
+            ull* w = p.gtab + (1ull << p.log2cap) * (ull)p.slot_words;
+            if (ld_volatile(w) == 0) *reinterpret_cast<volatile ull*>(w) = 1ull;
+            merge_words(w + p.st[0].word, K_COUNT, 1, 0);
+            merge_words(w + p.st[1].word, KIND, c0, c1);
+            return;
+        }
+        uint32_t h = ((uint32_t)g * 0x9E3779B1u) >> (32 - p.smem_log2);
+        volatile ull* vk = sk;
+        int sl = -1;
+        for (int i = 0; i < SMEM_PROBES; ++i) {
+            const ull k = vk[h];
+            if (k == stored) {
+                sl = (int)h;
+                break;
+            }
+            if (k == 0) {
+                if (*reinterpret_cast<volatile uint32_t*>(&s_fill) >= p.smem_fill) break;
+                const ull old = atomicCAS(&sk[h], 0ull, stored);
+                if (old == 0) atomicAdd(&s_fill, 1u);
+                if (old == 0 || old == stored) {
+                    sl = (int)h;
+                    break;
+                }
+            }
+            h = (h + 1) & (C - 1);
+        }
+        if (sl >= 0) {
+            ull* w = sw + (uint32_t)sl * (uint32_t)SW;
+            merge_words_smem(w + w0, K_COUNT, 1, 0, true);
+            merge_words_smem(w + w1, KIND, c0, c1, true);
+        } else {
+            const int64_t gs = g_find_insert(p, stored, inserts);
+            if (gs < 0) {
+                look = true;
+                return;
+            }
+            ull* w = p.gtab + (ull)gs * p.slot_words;
+            merge_words(w + p.st[0].word, K_COUNT, 1, 0);
+            merge_words(w + p.st[1].word, KIND, c0, c1);
+        }
+    };
+    KT nk[U];
+    uint32_t base = blockIdx.x * tile + threadIdx.x;  // row of u = 0
+#pragma unroll
+    for (int u = 0; u < U; ++u) nk[u] = base + u * blockDim.x < n ? __ldcs(keys + base + u * blockDim.x) : (KT)0;
+    for (uint32_t b = blockIdx.x * tile; b < n; b += step, base += step) {
+        ull key[U];
+        JoinBlock s[U];
+        ull lo[U], hi[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            key[u] = ~(ull)(ll)nk[u];  // (as stored)
+            s[u] = join_block(p.jslots, join_home(key[u], p.jlog2cap));
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t r = base + u * blockDim.x;
+            lo[u] = hi[u] = 0;
+            if (r >= n) continue;
+            const uint64_t at = p.row_begin + r;
+            if constexpr (KIND == K_SUM_D64) {
+                const ulonglong2 v = __ldcs(reinterpret_cast<const ulonglong2*>(p.st[1].col) + at);
+                lo[u] = v.x;
+                hi[u] = v.y;
+            } else if constexpr (KIND == K_SUM_I64) {
+                lo[u] = __ldcs(reinterpret_cast<const ull*>(p.st[1].col) + at);
+            } else {
+                lo[u] = (ull)(ll)__ldcs(reinterpret_cast<const int32_t*>(p.st[1].col) + at);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t r = base + step + u * blockDim.x;
+            nk[u] = (b + step < n && r < n) ? __ldcs(keys + r) : (KT)0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (base + u * blockDim.x >= n) continue;
+            ull w;
+            // (a full home block without the key: the rest of its chain; so
+            // too the key whose complement is 0, which has a slot of its own)
+            if (!join_step(s[u], key[u], w) || key[u] == 0) w = join_lookup(p.jslots, p.jlog2cap, ~key[u]);
+            if (w != ~0ull) fold((int32_t)(uint32_t)w, lo[u], (ll)hi[u] == ((ll)lo[u] >> 63));
+        }
+        // Publish new global groups and see whether the table must grow: at
+        // once where this warp met either, else now and then (the check reads
+        // the status word, a round trip).
+        const bool now = __any_sync(0xffffffffu, look || inserts != 0) || (++rounds & 15u) == 0;
+        look = false;
+        if (now && gb_warp_epilogue(p, inserts, pending)) break;
+    }
+    pending += __reduce_add_sync(0xffffffffu, inserts);
+    gb_warp_flush_pending(p, pending);
+    gb_flush_absbits(p, absbits);
+    __syncthreads();
+    gb_flush_shared(p, sk, sw, C);
+}
+
 // ---------------------------------------------------------------------------
 // Staged aggregation kernel.
 //
@@ -1001,6 +1144,20 @@ AggKernel agg_kernel_for(int spec, int n_st) {
     }
 }
 
+// The dense join kernel for a plan, or nullptr: COUNT(*) and one SUM, no
+// validity, a shared table, row numbers below 2^31 with a step to spare.
+AggKernel join_lean_kernel_for(const GbParams& p) {
+    if (!p.jslots || p.jkvalid || !p.smem_log2 || p.n_rows >= (1ull << 31) || (p.spec != 3 && p.spec != 4 && p.spec != 7) ||
+        p.st[1].valid || p.warp_agg)
+        return nullptr;
+    const bool k32 = p.jkdt == BOLT_I32;
+    switch (p.spec) {
+    case 3: return k32 ? gb_join_lean_kernel<int32_t, Spec3, 2> : gb_join_lean_kernel<ll, Spec3, 2>;
+    case 4: return k32 ? gb_join_lean_kernel<int32_t, Spec4, 2> : gb_join_lean_kernel<ll, Spec4, 2>;
+    default: return k32 ? gb_join_lean_kernel<int32_t, Spec7, 2> : gb_join_lean_kernel<ll, Spec7, 2>;
+    }
+}
+
 BatchKernel batch_kernel_for(int spec, int max_st) {
     switch (spec) {
     case 1: return gb_batch_agg_kernel<4, 4, Spec1>;
@@ -1503,7 +1660,8 @@ static bolt_status gb_agg_one(bolt_ctx* ctx, GbPlan* pl, cudaStream_t s, uint32_
         }
         tiles = std::max<uint64_t>(p.n_rows / stg.tile_rows, 1);
     } else {
-        kfn = agg_kernel_for(p.spec, p.n_st);
+        kfn = join_lean_kernel_for(p);
+        if (!kfn) kfn = agg_kernel_for(p.spec, p.n_st);
         tiles = (p.n_rows + tile - 1) / tile;
     }
     int per_sm = 1;
