@@ -135,6 +135,7 @@ struct SortArgs {
     uint32_t loc_range;    // rows of one work item of the local step
     uint32_t* tile_ctr;    // NPASS + 2 (the last two: the local step's items, long runs found)
     LongRun* longs;
+    uint32_t max_longs;
     uint32_t* status;
 };
 
@@ -1063,7 +1064,7 @@ __global__ void __launch_bounds__(LOC_BLOCK) sort_long_kernel(const __grid_const
     uint32_t* bins = reinterpret_cast<uint32_t*>(skey + CAP);
     uint32_t* spay = bins + LOC_WORDS;
     uint16_t* ia = reinterpret_cast<uint16_t*>(spay + CAP);
-    const uint32_t runs = a.tile_ctr[KeyTraits<K>::NPASS + 1];
+    const uint32_t runs = min(a.tile_ctr[KeyTraits<K>::NPASS + 1], a.max_longs);
     for (uint32_t r = blockIdx.x; r < runs; r += gridDim.x) {
         const LongRun run = a.longs[r];
         const SegDesc& d = seg_desc(a, (int)run.sg);
@@ -1196,7 +1197,9 @@ __global__ void __launch_bounds__(LOC_BLOCK, 2) sort_local_kernel(const __grid_c
                     const uint64_t at = run_start_from<K>(kin, pos + win, n, sh);
                     if (lane == 0) {
                         s_lim[0] = at;
-                        a.longs[atomicAdd(&a.tile_ctr[KeyTraits<K>::NPASS + 1], 1u)] = LongRun{pos, at, (ull)sg};
+                        const uint32_t q = atomicAdd(&a.tile_ctr[KeyTraits<K>::NPASS + 1], 1u);
+                        if (q < a.max_longs) a.longs[q] = LongRun{pos, at, (ull)sg};
+                        else atomicOr(a.status, ST_FLAG_TIMEOUT);  // only reachable after a look-back timeout
                     }
                 }
                 __syncthreads();
@@ -1391,7 +1394,8 @@ bolt_status run_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
     a.lookback = (uint32_t*)arena_alloc(ctx, 2 * a.lb_stride * 4);
     a.tile_ctr = (uint32_t*)arena_alloc(ctx, 64);
     constexpr uint64_t LOC_CAP = (uint64_t)LOC_BLOCK * KeyTraits<K>::LOC_ITEMS;
-    a.longs = (LongRun*)arena_alloc(ctx, (sum_n / LOC_CAP + 1) * sizeof(LongRun));
+    a.max_longs = (uint32_t)(sum_n / LOC_CAP + 1);
+    a.longs = (LongRun*)arena_alloc(ctx, a.max_longs * sizeof(LongRun));
     a.status = ctx->d_status;
     if (!a.longs || (many && (!d_segs || !d_begins)) || !a.kA || !a.kB || !a.pA || !a.pB || !a.hist || !a.digit_base || !a.plan ||
         !a.lookback || !a.tile_ctr)
