@@ -539,7 +539,7 @@ def w_join_groupby(c: Ctx):
     probe_k = kms[1::2] if len(kms) >= 2 else kms
     alg_probe = npr * 24
     alg = nb * 12 + npr * 24
-    line = base_line(c, ms, npr, alg_probe, probe_k, "gb_agg_kernel (join lookup source)", "join_groupby",
+    line = base_line(c, ms, npr, alg_probe, probe_k, "gb_join_lean_kernel", "join_groupby",
                      {"workload": "hash inner join then aggregate: build 10M unique shuffled int64 keys + int32 g; "
                                   "probe 200M int64 fk (90% match), Decimal128(15,2) amount; GROUP BY g SUM, COUNT(*)",
                       "build_rows": nb, "probe_rows": npr, "algorithmic_bytes_step": alg,
@@ -587,11 +587,11 @@ def w_sort(c: Ctx, kind: str):
         n = a.sort_rows
         keys = np.empty(n, np.int64)
         dg._chunked(n, lambda a, b: keys.__setitem__(slice(a, b), dg.uniform_u64(4, 31, b - a, a).view(np.int64)))
-        dt, kb, np_ = "i64", 8, 8
+        dt, kb = "i64", 8
     else:
         n = a.sortf_rows
         keys = dg.sort_f32(n, seed=5)
-        dt, kb, np_ = "f32", 4, 4
+        dt, kb = "f32", 4
     col = c.bolt.Column(torch.from_numpy(keys).to(c.dev), dt)
     perm = torch.empty(n, dtype=torch.int32, device=c.dev)
     abi = importlib.import_module("craton_bolt_b200._abi")
@@ -607,12 +607,13 @@ def w_sort(c: Ctx, kind: str):
         return int(c.lib.bolt_ctx_last_launches(c.eng._ctx))
 
     ms, launches, kms, clocks = c.timed(step, a.steps, a.warmup)
-    # pass accounting: histogram reads keys once; each 8-bit pass reads and
-    # writes (key + u32 payload); the first pass reads only the key, the last
-    # writes only the payload.
-    passes = np_
-    alg = n * (kb + kb + (passes - 2) * 2 * (kb + 4) + (kb + kb + 4) + (kb + 4 + 4))
-    line = base_line(c, ms, n, alg, kms, "sort (histogram + passes)", f"sort_{kind}",
+    # pass accounting for the short schedule these spread-out keys get: the
+    # histogram reads keys once; two 8-bit passes read and write (key + u32
+    # payload), the first reading only the key; the local step reads both and
+    # writes the payload.
+    passes = 2
+    alg = n * (kb + (kb + kb + 4) + 2 * (kb + 4) + (kb + 4 + 4))
+    line = base_line(c, ms, n, alg, kms, "sort (histogram, two digit passes, local step)", f"sort_{kind}",
                      {"workload": f"ORDER BY radix sort: {n} {dt} keys" +
                                   (" uniform over the full range" if kind == "i64" else
                                    " incl. negatives, +-0, +-inf, 0.1% NaN"),

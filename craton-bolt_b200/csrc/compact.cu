@@ -17,9 +17,10 @@
 // on 16-byte boundaries, the usual case) has one thread stage every column's
 // tile into shared memory with bulk copies (cp.async.bulk) completing on an
 // mbarrier, and evaluates the WHERE conjuncts on the staged values.
-// compact_kernel handles everything else (unaligned columns, wide rows, the
-// row-id-only form ORDER BY uses for its NULL split) with per-element
-// asynchronous copies or direct loads.
+// compact_kernel handles everything else (unaligned columns, wide rows,
+// row-id lists) with per-element asynchronous copies or direct loads. The
+// NULL split of ORDER BY has kernels of its own (split_count_kernel,
+// split_write_kernel).
 //
 // Large bulk-staged inputs take a two-pass form instead: in one pass a CTA
 // waits for its predecessors' counts, and while warp 0 looks back the other

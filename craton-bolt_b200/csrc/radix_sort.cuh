@@ -1,5 +1,6 @@
-// radix_sort.cuh — onesweep LSD radix sort (8-bit digits, decoupled look-back)
-// over one or many independent segments in the same launches.
+// radix_sort.cuh — stable radix sort (8-bit digits, decoupled look-back, a
+// shared-memory step after the top digits) over one or many independent
+// segments in the same launches.
 #pragma once
 
 #include <vector>
