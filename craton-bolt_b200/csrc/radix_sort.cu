@@ -744,22 +744,17 @@ __device__ __forceinline__ uint64_t run_start_from(const K* keys, uint64_t p, ui
     return hi;
 }
 
-// Stable LSD radix sort of the rows [s, e) by one CTA, tile after tile, over
-// the digits that vary among them; the sorted payloads go to `out`. For the
-// rare runs longer than a window. It orders row numbers, in the
-// other ping-pong buffer's memory, and leaves the rows where they are.
-// src_in_a: which buffer holds the rows; cnt: LOC_NW * 256 words; base: 256
-// words.
+// Stable LSD radix sort of len rows (keys kx, payloads px) by one CTA, tile
+// after tile, over the digits that vary among them; the sorted payloads go to
+// `out`, those from gap_at on `gap` places further. For the rare runs longer
+// than a window. It orders row numbers, in ix and iy (len words each), and
+// leaves the rows where they are. cnt: LOC_NW * 256 words; base: 256 words.
 template <typename K>
-__device__ __forceinline__ void local_serial_sort(K* kA, K* kB, uint32_t* pA, uint32_t* pB, bool src_in_a, uint64_t s,
-                                               uint64_t e, uint32_t* out, uint32_t* cnt, uint32_t* base, ull* red) {
+__device__ __forceinline__ void local_serial_sort(const K* kx, const uint32_t* px, uint32_t* ix, uint32_t* iy, uint64_t len,
+                                               uint32_t* out, uint64_t gap_at, uint64_t gap, uint32_t* cnt, uint32_t* base,
+                                               ull* red) {
     constexpr int NP = KeyTraits<K>::NPASS;
     const int t = threadIdx.x, w = t >> 5, lane = t & 31;
-    const uint64_t len = e - s;
-    const K* kx = (src_in_a ? kA : kB) + s;
-    const uint32_t* px = (src_in_a ? pA : pB) + s;
-    uint32_t* ix = reinterpret_cast<uint32_t*>((src_in_a ? kB : kA) + s);
-    uint32_t* iy = (src_in_a ? pB : pA) + s;
     bool first = true;  // the order so far is the identity
     ull vary = 0;
     const K k0 = kx[0];
@@ -839,7 +834,7 @@ __device__ __forceinline__ void local_serial_sort(K* kA, K* kB, uint32_t* pA, ui
         iy = it;
         first = false;
     }
-    for (uint64_t i = t; i < len; i += LOC_BLOCK) out[s + i] = px[first ? (uint32_t)i : ix[i]];
+    for (uint64_t i = t; i < len; i += LOC_BLOCK) out[i + (i >= gap_at ? gap : 0)] = px[first ? (uint32_t)i : ix[i]];
     __syncthreads();
 }
 
@@ -975,20 +970,25 @@ __device__ __noinline__ void local_radix_sort(const K* skey, const uint32_t* spa
     __syncthreads();
 }
 
-// A run [s, e) longer than a window in which one value is so frequent that
-// the rows of any other fit a window: a sweep counts the rows below and equal
-// to it, a second one writes the equal rows' payloads in place and collects
-// the others, in order, at skey / spay, where local_radix_sort orders them
-// around the gap. False (nothing written) when no value is that frequent.
+// A run longer than a window (len rows at kin / pin) in which one value is
+// frequent: a sweep counts the rows below and equal to it, a second one writes
+// the equal rows' payloads in place and collects the others, in order, to be
+// sorted around the gap: at skey / spay by local_radix_sort where they fit a
+// window, else in the run's part of the other buffer (kalt / palt) by
+// local_serial_sort, with the run's own part, read for the last time, for its
+// row numbers. So a run costs two sweeps and the sort of its other rows,
+// however often its frequent value occurs (2^28 hashes with 1 % zeros and
+// 20,000 ids beside them: 39.0 ms with the whole run in local_serial_sort,
+// 10.9 ms). False (nothing written) when no
+// value is a quarter of a sample.
 template <typename K>
-__device__ __forceinline__ bool local_hot_run(const K* kin, const uint32_t* pin, uint64_t s, uint64_t e, uint32_t cap, K* skey,
-                                           uint32_t* spay, uint16_t* ia, uint32_t act, K lo, int bits, uint32_t* out,
-                                           uint32_t* cnt, uint32_t* wsum, ull* red) {
+__device__ __forceinline__ bool local_hot_run(K* kin, uint32_t* pin, K* kalt, uint32_t* palt, uint64_t len, uint32_t cap,
+                                           K* skey, uint32_t* spay, uint16_t* ia, uint32_t act, K lo, int bits,
+                                           uint32_t* out, uint32_t* cnt, uint32_t* base, uint32_t* wsum, ull* red) {
     constexpr int U = 8;
     const int t = threadIdx.x, w = t >> 5, lane = t & 31;
-    const uint64_t len = e - s;
     // Candidate: the most frequent of 32 samples (every warp finds the same).
-    const K mine = kin[s + (len / 32) * (uint32_t)lane + len / 64];
+    const K mine = kin[(len / 32) * (uint32_t)lane + len / 64];
     const uint32_t same = (uint32_t)__popc(__match_any_sync(0xffffffffu, mine));
     const uint32_t best = __reduce_max_sync(0xffffffffu, same);
     if (best < 8) return false;
@@ -999,7 +999,7 @@ __device__ __forceinline__ bool local_hot_run(const K* kin, const uint32_t* pin,
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const uint64_t i = i0 + (uint64_t)u * LOC_BLOCK;
-            k[u] = i < len ? kin[s + i] : ~(K)0;
+            k[u] = i < len ? kin[i] : ~(K)0;
             if (i < len) {
                 below += k[u] < hot;
                 equal += k[u] == hot;
@@ -1008,7 +1008,10 @@ __device__ __forceinline__ bool local_hot_run(const K* kin, const uint32_t* pin,
     }
     below = block_sum(below, red);
     equal = block_sum(equal, red);
-    if (len - equal > cap) return false;
+    const uint64_t n_rest = len - equal;
+    const bool fits = n_rest <= cap;
+    K* const krest = fits ? skey : kalt;
+    uint32_t* const prest = fits ? spay : palt;
     uint64_t rest = 0;  // rows of other values before the tile
     for (uint64_t t0 = 0; t0 < len; t0 += LOC_BLOCK * U) {
         // Warp w's part: rows t0 + w * 32 * U + [0, 32 * U), 32 at a time.
@@ -1017,8 +1020,8 @@ __device__ __forceinline__ bool local_hot_run(const K* kin, const uint32_t* pin,
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const uint64_t i = t0 + (uint64_t)(w * U + u) * 32 + lane;
-            k[u] = i < len ? kin[s + i] : hot;
-            pay[u] = i < len ? pin[s + i] : 0u;
+            k[u] = i < len ? kin[i] : hot;
+            pay[u] = i < len ? pin[i] : 0u;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -1037,10 +1040,10 @@ __device__ __forceinline__ bool local_hot_run(const K* kin, const uint32_t* pin,
             if (i < len) {
                 const uint64_t others = rest + before + __popc(me[u] & lanemask_lt());
                 if ((me[u] >> lane) & 1u) {
-                    skey[others] = k[u];
-                    spay[others] = pay[u];
+                    krest[others] = k[u];
+                    prest[others] = pay[u];
                 } else {
-                    out[s + below + (i - others)] = pay[u];
+                    out[below + (i - others)] = pay[u];
                 }
             }
             before += __popc(me[u]);
@@ -1048,8 +1051,11 @@ __device__ __forceinline__ bool local_hot_run(const K* kin, const uint32_t* pin,
         rest += all;
     }
     __syncthreads();
-    local_radix_sort<K>(skey, spay, ia, ia + cap, (uint32_t)(len - equal), act, lo, bits, out + s, (uint32_t)below, equal, cnt,
-                        wsum, red);
+    if (fits)
+        local_radix_sort<K>(skey, spay, ia, ia + cap, (uint32_t)n_rest, act, lo, bits, out, (uint32_t)below, equal, cnt, wsum,
+                            red);
+    else
+        local_serial_sort<K>(kalt, palt, reinterpret_cast<uint32_t*>(kin), pin, n_rest, out, below, equal, cnt, base, red);
     return true;
 }
 
@@ -1069,18 +1075,18 @@ __global__ void __launch_bounds__(LOC_BLOCK) sort_long_kernel(const __grid_const
         const LongRun run = a.longs[r];
         const SegDesc& d = seg_desc(a, (int)run.sg);
         const SegPlan plan = a.plan[run.sg];
-        K* kA = (K*)a.kA + d.buf_off;
-        K* kB = (K*)a.kB + d.buf_off;
-        uint32_t* pA = a.pA + d.buf_off;
-        uint32_t* pB = a.pB + d.buf_off;
         const bool in_a = (__popc(plan.sched) & 1) != 0;
-        const K* kin = in_a ? kA : kB;
+        const uint64_t at = d.buf_off + run.s, len = run.e - run.s;
+        K* kin = (K*)(in_a ? a.kA : a.kB) + at;
+        K* kalt = (K*)(in_a ? a.kB : a.kA) + at;
+        uint32_t* pin = (in_a ? a.pA : a.pB) + at;
+        uint32_t* palt = (in_a ? a.pB : a.pA) + at;
+        uint32_t* out = d.payload_out + run.s;
         const Packer pack(plan.act, (int)sizeof(K));
         const int psh = 8 * (__popc(plan.act) - __popc(plan.sched));
-        const K lo = (K)((pack(kin[run.s]) >> psh) << psh);
-        if (!local_hot_run<K>(kin, in_a ? pA : pB, run.s, run.e, CAP, skey, spay, ia, plan.act, lo, psh, d.payload_out, bins,
-                              s_wsum, red))
-            local_serial_sort<K>(kA, kB, pA, pB, in_a, run.s, run.e, d.payload_out, bins, s_base, red);
+        const K lo = (K)((pack(kin[0]) >> psh) << psh);
+        if (!local_hot_run<K>(kin, pin, kalt, palt, len, CAP, skey, spay, ia, plan.act, lo, psh, out, bins, s_base, s_wsum, red))
+            local_serial_sort<K>(kin, pin, reinterpret_cast<uint32_t*>(kalt), palt, len, out, len, 0, bins, s_base, red);
         __syncthreads();
     }
 }

@@ -1,0 +1,56 @@
+"""Runs of equal top digits longer than the local step's window, mostly one value among others of its run: the order
+against numpy's stable argsort, and the time against keys for which every digit gets a pass."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _full(rng, n):
+    return rng.integers(-(1 << 63), (1 << 63) - 1, n, dtype=np.int64)
+
+
+def _sort(bolt, engine, v, reps=1):
+    """(permutation, least device time in ms)"""
+    col = bolt.col(v).to("cuda")
+    ms = []
+    for _ in range(reps):
+        perm = engine.sort_indices([col])
+        ms.append(engine.last_device_ms)
+    return perm.cpu().numpy().view(np.uint32), min(ms)
+
+
+def _hot(rng, n, hot, others):
+    """Uniform keys, of which `hot` are 0 and `others` are ids that share its top three bytes."""
+    v = _full(rng, n)
+    at = rng.permutation(n)
+    v[at[:hot]] = 0
+    v[at[hot:hot + others]] = rng.integers(1, 1 << 40, others)
+    return v
+
+
+# 5,120 rows of other values: one window of 64-bit keys.
+@pytest.mark.parametrize("others", [5119, 5120, 5121, 8000])
+@pytest.mark.parametrize("n,hot", [(3_000_017, 40_000), (1 << 24, 200_001)])
+def test_others_around_one_window(bolt, engine, n, hot, others):
+    v = _hot(np.random.default_rng(others), n, hot, others)
+    got, _ = _sort(bolt, engine, v)
+    assert np.array_equal(got, np.argsort(v, kind="stable"))
+
+
+def test_no_slower_than_every_digit(bolt, engine):
+    """2^24 keys, 1.2 % of one value and 8,000 ids beside it, against keys that crowd (one pass per digit). The bound
+    is the schedule's purpose: it is taken to be faster than the passes it leaves out."""
+    n = 1 << 24
+    rng = np.random.default_rng(1)
+    v = _hot(rng, n, 200_000, 8_000)
+    got, ms = _sort(bolt, engine, v, 5)
+    assert np.array_equal(got, np.argsort(v, kind="stable"))
+    crowded = _full(rng, n)
+    crowded[::2] = (crowded[::2] & 0xFFFFFFFFFF) + (5 << 40)
+    got, all_ms = _sort(bolt, engine, crowded, 5)
+    assert np.array_equal(got, np.argsort(crowded, kind="stable"))
+    assert ms <= all_ms
