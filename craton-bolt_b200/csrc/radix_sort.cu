@@ -63,7 +63,7 @@ constexpr int LOC_NW = LOC_BLOCK / 32;
 constexpr int LOC_BINS_LOG2 = 14;  // bins of the local step, counted in bytes
 constexpr int LOC_WORDS = (1 << LOC_BINS_LOG2) / 4;
 // Keys one bin may hold (a byte counts them): every key is compared with the
-// others of its bin, so chunks with longer ones take local_radix_sort.
+// others of its bin, so chunks with longer ones take local_merge_sort.
 constexpr uint32_t LOC_BIN_MAX = 32;
 constexpr int LOC_SER_ROUNDS = 4;  // 32-key rounds per warp and tile of the serial path
 
@@ -859,121 +859,94 @@ struct Packer {
     __device__ __forceinline__ uint32_t operator()(uint32_t k) const { return __byte_perm(k, 0u, lo); }
 };
 
-// One stable counting pass of the crowded-chunk sort over the row numbers
-// src -> dst (identity: src is 0, 1, 2, ...), by digit(row).
-template <int ITEMS, class Digit>
-__device__ __forceinline__ void local_pass(const uint16_t* src, uint16_t* dst, bool identity, uint32_t len, uint32_t* cnt,
-                                           uint32_t* wsum, Digit digit) {
-    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
-    for (int i = t; i < LOC_NW * 256; i += LOC_BLOCK) cnt[i] = 0;
-    __syncthreads();
-    uint32_t rd[ITEMS];  // row | digit << 16
-#pragma unroll
-    for (int r = 0; r < ITEMS; ++r) {
-        const uint32_t p = (uint32_t)(w * ITEMS + r) * 32 + lane;
-        rd[r] = 0;
-        if (p < len) {
-            const uint32_t id = identity ? p : src[p], dg = digit(id);
-            rd[r] = id | (dg << 16);
-            atomicAdd(&cnt[w * 256 + dg], 1u);
-        }
-    }
-    __syncthreads();
-    uint32_t run = 0, x = 0;
-    if (t < 256) {
-        for (int ww = 0; ww < LOC_NW; ++ww) run += cnt[ww * 256 + t];
-        x = run;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) wsum[w] = x;
-    }
-    __syncthreads();
-    if (t < 256) {
-        uint32_t off = x - run;
-        for (int i = 0; i < w; ++i) off += wsum[i];
-        for (int ww = 0; ww < LOC_NW; ++ww) {
-            const uint32_t c = cnt[ww * 256 + t];
-            cnt[ww * 256 + t] = off;
-            off += c;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < ITEMS; ++r) {
-        const uint32_t p = (uint32_t)(w * ITEMS + r) * 32 + lane;
-        const bool in = p < len;
-        const uint32_t dg = rd[r] >> 16;
-        uint32_t peers = __ballot_sync(0xffffffffu, in);
-#pragma unroll
-        for (int bit = 0; bit < 8; ++bit) {
-            const uint32_t on = (dg >> bit) & 1u;
-            const uint32_t bal = __ballot_sync(0xffffffffu, on);
-            peers &= on ? bal : ~bal;
-        }
-        uint32_t b = 0;
-        if (in) b = cnt[w * 256 + dg];
-        __syncwarp();
-        if (in) {
-            if (lane == 31 - __clz(peers)) cnt[w * 256 + dg] = b + __popc(peers);
-            dst[b + __popc(peers & lanemask_lt())] = (uint16_t)(rd[r] & 0xFFFFu);
-        }
-        __syncwarp();
-    }
-    __syncthreads();
-}
-
 // Sorts a chunk whose keys crowd into too few bins (repeated keys, or gaps
 // between clusters), in shared memory: skey holds its keys in chunk order,
-// spay the payloads. A stable radix sort of the row numbers by the leading 16
-// bits of the keys' range settles the repeated keys; where it does not leave
-// the keys in order, all varying digits are sorted.
+// spay the payloads; payloads from gap_at on go `gap` places further. A stable
+// merge sort of the row numbers (ia, ib): each thread sorts LOC_ITEMS
+// neighbours in registers, then pairs of lists are merged, each thread its own
+// LOC_ITEMS outputs of a pair from where a binary search says they begin. Its
+// cost is the same for all keys, and short, since the grid ends with its
+// slowest chunk (2M floats with 2,000 of each special value: local step 64 us
+// with two to ten counting passes here, 50 us; 32 us without such values).
 template <typename K>
-__device__ __noinline__ void local_radix_sort(const K* skey, const uint32_t* spay, uint16_t* ia, uint16_t* ib, uint32_t len,
-                                              uint32_t act, K lo, int bits, uint32_t* out, uint32_t gap_at, uint64_t gap,
-                                              uint32_t* cnt, uint32_t* wsum, ull* red) {
-    constexpr int ITEMS = KeyTraits<K>::LOC_ITEMS;
-    const int t = threadIdx.x;
-    const Packer pack(act, (int)sizeof(K));
-    const int top = bits > 16 ? bits - 16 : 0;
-    local_pass<ITEMS>(ia, ia, true, len, cnt, wsum, [&](uint32_t i) { return (uint32_t)((K)(pack(skey[i]) - lo) >> top) & 0xFFu; });
-    local_pass<ITEMS>(ia, ib, false, len, cnt, wsum,
-                      [&](uint32_t i) { return (uint32_t)((K)(pack(skey[i]) - lo) >> top >> 8) & 0xFFu; });
-    uint16_t* cur = ib;
-    if (bits > 16) {
-        bool ok = true;
-        for (uint32_t p = t + 1; p < len; p += LOC_BLOCK) ok = ok && skey[ib[p - 1]] <= skey[ib[p]];
-        if (!__syncthreads_and(ok)) {
-            ull vary = 0;
-            for (uint32_t p = t; p < len; p += LOC_BLOCK) vary |= (ull)(skey[p] ^ skey[0]);
+__device__ __noinline__ void local_merge_sort(const K* skey, const uint32_t* spay, uint16_t* ia, uint16_t* ib, uint32_t len,
+                                              uint32_t* out, uint32_t gap_at, uint64_t gap) {
+    constexpr uint32_t ITEMS = KeyTraits<K>::LOC_ITEMS;
+    const uint32_t t = threadIdx.x;
+    {
+        K k[ITEMS];
+        uint32_t id[ITEMS];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) vary |= __shfl_xor_sync(0xffffffffu, vary, o);
-            if ((t & 31) == 0) red[t >> 5] = vary;
-            __syncthreads();
-            for (int i = 0; i < LOC_NW; ++i) vary |= red[i];
-            uint16_t *src = ia, *dst = ib;
-            bool identity = true;
-            for (int p = 0; p < KeyTraits<K>::NPASS; ++p) {
-                if (((vary >> (8 * p)) & 0xFFull) == 0) continue;
-                local_pass<ITEMS>(src, dst, identity, len, cnt, wsum, [&](uint32_t i) { return digit_of<K>(skey[i], 8 * p); });
-                identity = false;
-                uint16_t* const x = src;
-                src = dst;
-                dst = x;
-            }
-            cur = src;
+        for (uint32_t j = 0; j < ITEMS; ++j) {
+            id[j] = t * ITEMS + j;
+            k[j] = id[j] < len ? skey[id[j]] : ~(K)0;  // (rows past the end stay behind equal keys)
         }
+#pragma unroll
+        for (uint32_t r = 0; r < ITEMS; ++r) {  // odd-even transposition: neighbours only, so it is stable
+#pragma unroll
+            for (uint32_t j = r & 1; j + 1 < ITEMS; j += 2) {
+                const bool sw = k[j] > k[j + 1];
+                const K a = sw ? k[j + 1] : k[j], b = sw ? k[j] : k[j + 1];
+                const uint32_t x = sw ? id[j + 1] : id[j], y = sw ? id[j] : id[j + 1];
+                k[j] = a;
+                k[j + 1] = b;
+                id[j] = x;
+                id[j + 1] = y;
+            }
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < ITEMS; ++j)
+            if (t * ITEMS + j < len) ia[t * ITEMS + j] = (uint16_t)id[j];
     }
-    for (uint32_t p = t; p < len; p += LOC_BLOCK) out[p + (p >= gap_at ? gap : 0)] = spay[cur[p]];
+    __syncthreads();
+    uint16_t *src = ia, *dst = ib;
+    for (uint32_t w = ITEMS; w < len; w *= 2) {
+        // Lists a (na rows) and b (nb rows) of the thread's pair; its outputs
+        // are [d, d + ITEMS) of the merged list.
+        const uint32_t per = 2 * w / ITEMS, base = (t / per) * 2 * w, d = (t & (per - 1)) * ITEMS;
+        const uint32_t mid = min(base + w, len), end = min(base + 2 * w, len);
+        if (base + d < len) {
+            const uint16_t *a = src + base, *b = src + mid;
+            const uint32_t na = mid - base, nb = end - mid;
+            const uint32_t stop = min(d + ITEMS, na + nb);
+            if (nb == 0 || skey[a[na - 1]] <= skey[b[0]]) {
+                // In order already (a chunk's runs are, and equal keys):
+                // the two lists, one after the other.
+                for (uint32_t o = d; o < stop; ++o) dst[base + o] = a[o];
+            } else {
+                uint32_t lo = d > nb ? d - nb : 0, hi = min(d, na);
+                while (lo < hi) {  // rows of a before output d (a's come first among equal keys)
+                    const uint32_t m = (lo + hi) / 2;
+                    if (skey[a[m]] <= skey[b[d - 1 - m]]) lo = m + 1;
+                    else hi = m;
+                }
+                uint32_t i = lo, j = d - lo;
+                uint32_t x = i < na ? a[i] : 0, y = j < nb ? b[j] : 0;
+                K kx = skey[x], ky = skey[y];
+                for (uint32_t o = d; o < stop; ++o) {
+                    const bool from_a = j >= nb || (i < na && kx <= ky);
+                    dst[base + o] = (uint16_t)(from_a ? x : y);
+                    if (from_a) {
+                        if (++i < na) kx = skey[x = a[i]];
+                    } else {
+                        if (++j < nb) ky = skey[y = b[j]];
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        uint16_t* const z = src;
+        src = dst;
+        dst = z;
+    }
+    for (uint32_t p = t; p < len; p += LOC_BLOCK) out[p + (p >= gap_at ? gap : 0)] = spay[src[p]];
     __syncthreads();
 }
 
 // A run longer than a window (len rows at kin / pin) in which one value is
 // frequent: a sweep counts the rows below and equal to it, a second one writes
 // the equal rows' payloads in place and collects the others, in order, to be
-// sorted around the gap: at skey / spay by local_radix_sort where they fit a
+// sorted around the gap: at skey / spay by local_merge_sort where they fit a
 // window, else in the run's part of the other buffer (kalt / palt) by
 // local_serial_sort, with the run's own part, read for the last time, for its
 // row numbers. So a run costs two sweeps and the sort of its other rows,
@@ -983,8 +956,8 @@ __device__ __noinline__ void local_radix_sort(const K* skey, const uint32_t* spa
 // value is a quarter of a sample.
 template <typename K>
 __device__ __forceinline__ bool local_hot_run(K* kin, uint32_t* pin, K* kalt, uint32_t* palt, uint64_t len, uint32_t cap,
-                                           K* skey, uint32_t* spay, uint16_t* ia, uint32_t act, K lo, int bits,
-                                           uint32_t* out, uint32_t* cnt, uint32_t* base, uint32_t* wsum, ull* red) {
+                                           K* skey, uint32_t* spay, uint16_t* ia, uint32_t* out, uint32_t* cnt,
+                                           uint32_t* base, uint32_t* wsum, ull* red) {
     constexpr int U = 8;
     const int t = threadIdx.x, w = t >> 5, lane = t & 31;
     // Candidate: the most frequent of 32 samples (every warp finds the same).
@@ -1052,8 +1025,7 @@ __device__ __forceinline__ bool local_hot_run(K* kin, uint32_t* pin, K* kalt, ui
     }
     __syncthreads();
     if (fits)
-        local_radix_sort<K>(skey, spay, ia, ia + cap, (uint32_t)n_rest, act, lo, bits, out, (uint32_t)below, equal, cnt, wsum,
-                            red);
+        local_merge_sort<K>(skey, spay, ia, ia + cap, (uint32_t)n_rest, out, (uint32_t)below, equal);
     else
         local_serial_sort<K>(kalt, palt, reinterpret_cast<uint32_t*>(kin), pin, n_rest, out, below, equal, cnt, base, red);
     return true;
@@ -1082,10 +1054,7 @@ __global__ void __launch_bounds__(LOC_BLOCK) sort_long_kernel(const __grid_const
         uint32_t* pin = (in_a ? a.pA : a.pB) + at;
         uint32_t* palt = (in_a ? a.pB : a.pA) + at;
         uint32_t* out = d.payload_out + run.s;
-        const Packer pack(plan.act, (int)sizeof(K));
-        const int psh = 8 * (__popc(plan.act) - __popc(plan.sched));
-        const K lo = (K)((pack(kin[0]) >> psh) << psh);
-        if (!local_hot_run<K>(kin, pin, kalt, palt, len, CAP, skey, spay, ia, plan.act, lo, psh, out, bins, s_base, s_wsum, red))
+        if (!local_hot_run<K>(kin, pin, kalt, palt, len, CAP, skey, spay, ia, out, bins, s_base, s_wsum, red))
             local_serial_sort<K>(kin, pin, reinterpret_cast<uint32_t*>(kalt), palt, len, out, len, 0, bins, s_base, red);
         __syncthreads();
     }
@@ -1262,8 +1231,7 @@ __global__ void __launch_bounds__(LOC_BLOCK, 2) sort_local_kernel(const __grid_c
                 }
                 __syncthreads();
                 uint16_t* ia = reinterpret_cast<uint16_t*>(smeta);
-                local_radix_sort<K>(skey, spay, ia, ia + CAP, len, plan.act, lo, bits, d.payload_out + pos, len, 0, bins, s_wsum,
-                                    red);
+                local_merge_sort<K>(skey, spay, ia, ia + CAP, len, d.payload_out + pos, len, 0);
                 pos += len;
                 continue;
             }

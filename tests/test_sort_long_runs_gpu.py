@@ -54,3 +54,31 @@ def test_no_slower_than_every_digit(bolt, engine):
     got, all_ms = _sort(bolt, engine, crowded, 5)
     assert np.array_equal(got, np.argsort(crowded, kind="stable"))
     assert ms <= all_ms
+
+
+def test_crowded_window_costs_little(bolt, engine):
+    """One window whose keys crowd into a few bins, against uniform keys: a crowded chunk is one block's work, and the
+    grid ends with it."""
+    n = 5000
+    rng = np.random.default_rng(8)
+    v = _full(rng, n)
+    _, uniform_ms = _sort(bolt, engine, v, 25)
+    v[::2] = (v[::2] & 0xFFFFFF) + (5 << 40)
+    got, ms = _sort(bolt, engine, v, 25)
+    assert np.array_equal(got, np.argsort(v, kind="stable"))
+    print(f"crowded {ms * 1e3:.1f} us, uniform {uniform_ms * 1e3:.1f}")
+    assert ms <= 1.5 * uniform_ms
+
+
+# 5,120 rows: one window; 10 rows: what one thread sorts by itself.
+@pytest.mark.parametrize("n", [33, 5000, 5111, 5119, 5120])
+@pytest.mark.parametrize("values", [2, 90])
+def test_crowded_window(bolt, engine, n, values):
+    """Few values far apart and clusters around them, in one window: the bins are too long, the merge sort orders it."""
+    rng = np.random.default_rng(n * values)
+    v = rng.choice(_full(rng, values), n)
+    near = rng.random(n) < 0.5
+    v[near] ^= rng.integers(0, 64, near.sum())
+    for x in (v, v >> 40, (v >> 32).astype(np.int32)):
+        got, _ = _sort(bolt, engine, x)
+        assert np.array_equal(got, np.argsort(x, kind="stable"))
