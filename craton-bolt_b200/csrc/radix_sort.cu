@@ -76,6 +76,13 @@ template <> struct KeyTraits<uint32_t> {
     // Mean run length (share of its window) up to which it is used: 32-bit
     // keys drop two passes by it and lose that to runs past the window sooner.
     static constexpr double LOC_FULL = 0.8;
+    // The longest run let through: this share of the rows and half a window.
+    // One CTA sorts it, 16 ns a row (64-bit keys; 7 ns for 32-bit ones, fewer
+    // digits), and that is what the passes left out take for runs of 5,900,
+    // 9,200, 19,000 and 50,000 rows in 1, 3, 10 and 30M (32-bit keys: 5,500,
+    // 12,000 and 40,000 in 5, 20 and 60M). Near a window's length the sample's
+    // estimate is off by a third either way; the passes are the safe side.
+    static constexpr uint32_t LOC_RUN = 2000;
 };
 template <> struct KeyTraits<ull> {
     static constexpr int NPASS = 8;
@@ -83,6 +90,7 @@ template <> struct KeyTraits<ull> {
     static constexpr int TILE = SORT_BLOCK * ITEMS;
     static constexpr int LOC_ITEMS = 10;
     static constexpr double LOC_FULL = 0.9;
+    static constexpr uint32_t LOC_RUN = 600;
 };
 
 struct SegDesc {
@@ -205,10 +213,32 @@ __device__ __forceinline__ uint64_t seg_n(const SegDesc& d) {
     return n < d.n ? n : d.n;
 }
 
+// Key i of a segment's source, transformed.
+template <typename K>
+__device__ __forceinline__ K source_key(const SortArgs& a, const SegDesc& d, uint64_t i) {
+    return order_key(a.src, raw_key<K>(d.keys, a.indirect ? d.payload_in[i] : i), a.desc);
+}
+
+// Keys that sort_plan_kernel looks at, of a segment of n rows: as many as show
+// a mean run of CAP rows in some 250 pairs (m * m from n / 8), and as show a
+// run of n / LOC_RUN rows in a dozen; one a thread of its block costs no more
+// than a few. Part i of m equal parts gives the sample at sample_row(i).
+template <typename K>
+__device__ __forceinline__ uint32_t sample_count(uint64_t n) {
+    uint32_t m = 256;
+    auto more = [&](uint64_t mm) { return m < PLAN_BLOCK || mm < n / 8 || (m < PLAN_SAMPLES && mm < 2 * n); };
+    while (m < PLAN_SAMPLES && 4 * m <= n && more((uint64_t)m * m)) m *= 2;
+    return m;
+}
+__device__ __forceinline__ uint32_t sample_row(uint32_t i, uint32_t step) { return i * step + __umulhi(i * 2654435761u, step); }
+
 // Digit histograms of every segment. Bound by its shared-memory counter adds
 // (one per digit and key, about 7.5 lanes per SM and cycle; four copies of
 // every counter in neighbouring banks changed nothing). A CTA flushes its
-// counters once per segment it meets.
+// counters once per segment it meets. The rows in hand, it also leaves the
+// plan's samples at the start of the segment's first key buffer: gathered by
+// the plan's one CTA they cost a DRAM round trip per few hundred (5M 32-bit
+// keys, 4,096 samples: plan 18.1 us, 11.7 us with them at hand).
 template <typename K>
 __global__ void __launch_bounds__(HIST_BLOCK) sort_hist_kernel(const __grid_constant__ SortArgs a) {
     constexpr int NP = KeyTraits<K>::NPASS;
@@ -220,6 +250,7 @@ __global__ void __launch_bounds__(HIST_BLOCK) sort_hist_kernel(const __grid_cons
     if (blockIdx.x == 0 && threadIdx.x < NP + 2) a.tile_ctr[threadIdx.x] = 0;
     for (int i = threadIdx.x; i < NP * 256; i += blockDim.x) h[i] = 0;
     int cur = -1;
+    uint32_t smp = 0, smp_step = 1;  // samples of the segment, rows of one's part
     auto flush = [&]() {
         __syncthreads();
         uint32_t* gh = a.hist + (uint64_t)cur * NP * 256;
@@ -231,13 +262,18 @@ __global__ void __launch_bounds__(HIST_BLOCK) sort_hist_kernel(const __grid_cons
     };
     for (uint32_t item = blockIdx.x; item < a.total_hist_items; item += gridDim.x) {
         const int sg = seg_of(a.hist_begins, a.nseg, item);
-        if (sg != cur) {
+        const bool fresh = sg != cur;
+        if (fresh) {
             if (cur >= 0) flush();
             __syncthreads();
             cur = sg;
         }
         const SegDesc& d = seg_desc(a, sg);
         const uint64_t n = seg_n(d);
+        if (fresh) {
+            smp = n > LOC_BLOCK * KeyTraits<K>::LOC_ITEMS ? sample_count<K>(n) : 0u;
+            if (smp) smp_step = (uint32_t)n / smp;  // n < 2^30
+        }
         const uint64_t c0 = (uint64_t)(item - d.hist_begin) * HIST_CHUNK;
         const uint64_t c1 = c0 + HIST_CHUNK < n ? c0 + HIST_CHUNK : n;
         for (uint64_t i0 = c0 + threadIdx.x; i0 < c1; i0 += 4 * blockDim.x) {
@@ -256,14 +292,13 @@ __global__ void __launch_bounds__(HIST_BLOCK) sort_hist_kernel(const __grid_cons
                 for (int p = 0; p < NP; ++p) atomicAdd(&h[p * 256 + digit_of<K>(k, 8 * p)], 1u);
             }
         }
+        if (c0 >= n) continue;
+        for (uint32_t i = (uint32_t)c0 / smp_step + threadIdx.x; i < smp && (uint64_t)i * smp_step < c1; i += blockDim.x) {
+            const uint32_t r = sample_row(i, smp_step);
+            if (r >= c0 && r < c1) ((K*)a.kA + d.buf_off)[i] = source_key<K>(a, d, r);
+        }
     }
     if (cur >= 0) flush();
-}
-
-// Key i of a segment's source, transformed.
-template <typename K>
-__device__ __forceinline__ K source_key(const SortArgs& a, const SegDesc& d, uint64_t i) {
-    return order_key(a.src, raw_key<K>(d.keys, a.indirect ? d.payload_in[i] : i), a.desc);
 }
 
 // Sum of v over the block (every thread gets it); red holds one word per warp.
@@ -318,65 +353,71 @@ __device__ __forceinline__ void block_min_max(K& mn, K& mx, ull* red) {
 // the local step lets the value's rows through in one sweep. All of it only
 // steers the speed: the local step orders runs of any length.
 struct SampleRuns {
-    ull pairs;     // agreeing pairs
-    ull longest;   // most samples in one run
-    ull hottest;   // most samples of one value left out of the two
+    uint32_t pairs;     // agreeing pairs
+    uint32_t longest;   // most samples in one run
+    uint32_t hottest;   // most samples of one value left out of the two
 };
 
 // Counts the runs of equal key >> sh among the block's samples (cnt_s per
 // thread). tab: 32-bit hashes of the prefixes, mask + 1 slots, half empty;
 // cnt: samples | samples that differ from the slot's first << 16; fst: hash
-// of the slot's first key.
+// of the slot's first key. One block does this between two launches, so it is
+// all latency: one CAS a sample, then counts that wait for nothing, and one
+// round of reductions.
 template <typename K>
 __device__ __forceinline__ SampleRuns sample_runs(const K (&smp)[PLAN_PER], int cnt_s, int sh, uint32_t mask, uint32_t* tab,
-                                                  uint32_t* cnt, uint32_t* fst, ull* red) {
+                                                  uint32_t* cnt, uint32_t* fst, uint32_t* red) {
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i <= mask; i += PLAN_BLOCK) {
-        tab[i] = 0;
-        cnt[i] = 0;
-        fst[i] = 0;
+    for (uint32_t i = 4 * threadIdx.x; i <= mask; i += 4 * PLAN_BLOCK) {
+        *reinterpret_cast<uint4*>(tab + i) = make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4*>(cnt + i) = make_uint4(0, 0, 0, 0);
     }
     __syncthreads();
+    uint32_t at[PLAN_PER], own[PLAN_PER];
 #pragma unroll
     for (int u = 0; u < PLAN_PER; ++u) {
         if (u >= cnt_s) continue;
         const ull hp = (ull)(smp[u] >> sh) * 0x9E3779B97F4A7C15ull;
         const uint32_t sig = (uint32_t)(hp >> 32) | 1u;
-        const uint32_t own = (uint32_t)(((ull)smp[u] * 0xD6E8FEB86659FD93ull) >> 32) | 1u;
+        own[u] = (uint32_t)(((ull)smp[u] * 0xD6E8FEB86659FD93ull) >> 32);
         uint32_t h = (uint32_t)(hp >> 40) & mask;
         for (uint32_t probe = 0; probe <= mask; ++probe) {
             const uint32_t old = atomicCAS(&tab[h], 0u, sig);
-            if (old == 0 || old == sig) {
-                const uint32_t f = atomicCAS(&fst[h], 0u, own);
-                atomicAdd(&cnt[h], f == 0 || f == own ? 1u : 0x10001u);
-                break;
-            }
+            if (old == 0) fst[h] = own[u];
+            if (old == 0 || old == sig) break;
             h = (h + 1) & mask;
         }
+        at[u] = h;
     }
     __syncthreads();
-    ull pairs = 0;
-    uint32_t longest = 0, hottest = 0;
+#pragma unroll
+    for (int u = 0; u < PLAN_PER; ++u)
+        if (u < cnt_s) atomicAdd(&cnt[at[u]], fst[at[u]] == own[u] ? 1u : 0x10001u);
+    __syncthreads();
+    SampleRuns r{0, 0, 0};
     for (uint32_t i = threadIdx.x; i <= mask; i += PLAN_BLOCK) {
         const uint32_t all = cnt[i] & 0xFFFFu, other = cnt[i] >> 16, same = all - other;
         uint32_t c = all;
         if (same >= 4 && other * 4 <= all) {
             c = other + 1;
-            hottest = max(hottest, same);
+            r.hottest = max(r.hottest, same);
         }
-        pairs += (ull)c * (c ? c - 1 : 0) / 2;
-        longest = max(longest, c);
+        r.pairs += c * (c ? c - 1 : 0) / 2;
+        r.longest = max(r.longest, c);
     }
-    SampleRuns r;
-    r.pairs = block_sum(pairs, red);
-    longest = __reduce_max_sync(0xffffffffu, longest);
-    hottest = __reduce_max_sync(0xffffffffu, hottest);
+    // (pairs fit 32 bits: 8,192 samples have 33.5M)
+    r.pairs = __reduce_add_sync(0xffffffffu, r.pairs);
+    r.longest = __reduce_max_sync(0xffffffffu, r.longest);
+    r.hottest = __reduce_max_sync(0xffffffffu, r.hottest);
+    if ((threadIdx.x & 31) == 0) {
+        red[threadIdx.x >> 5] = r.pairs;
+        red[32 + (threadIdx.x >> 5)] = r.longest;
+        red[64 + (threadIdx.x >> 5)] = r.hottest;
+    }
     __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = (ull)longest << 32 | hottest;
-    __syncthreads();
-    const ull m = red[threadIdx.x & 31];
-    r.longest = __reduce_max_sync(0xffffffffu, (uint32_t)(m >> 32));
-    r.hottest = __reduce_max_sync(0xffffffffu, (uint32_t)m);
+    r.pairs = __reduce_add_sync(0xffffffffu, red[threadIdx.x & 31]);
+    r.longest = __reduce_max_sync(0xffffffffu, red[32 + (threadIdx.x & 31)]);
+    r.hottest = __reduce_max_sync(0xffffffffu, red[64 + (threadIdx.x & 31)]);
     return r;
 }
 
@@ -389,12 +430,28 @@ __global__ void __launch_bounds__(PLAN_BLOCK) sort_plan_kernel(const __grid_cons
     uint32_t* cnt = tab + 2 * PLAN_SAMPLES;                // 2 * PLAN_SAMPLES words
     uint32_t* fst = cnt + 2 * PLAN_SAMPLES;                // 2 * PLAN_SAMPLES words
     __shared__ uint32_t s_act;
-    __shared__ ull red[PLAN_BLOCK / 32];
+    static_assert(PLAN_BLOCK == 1024, "red: three words a warp, or a 64-bit one");
+    __shared__ ull red[48];
     const int sg = blockIdx.x;
     const SegDesc& d = seg_desc(a, sg);
     const uint64_t n = seg_n(d);
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     if (t == 0) s_act = 0;
+    const uint32_t m = sample_count<K>(n), step = (uint32_t)n / m;  // n < 2^30
+    // (On their way while the histograms are scanned.)
+    K smp[PLAN_PER];
+    int cnt_s = 0;
+    if (n > CAP) {
+#pragma unroll
+        for (int u = 0; u < PLAN_PER; ++u) {
+            const uint32_t i = (uint32_t)u * PLAN_BLOCK + t;
+            smp[u] = 0;
+            if (i < m) {
+                smp[u] = ((const K*)a.kA + d.buf_off)[i];
+                cnt_s = u + 1;
+            }
+        }
+    }
     __syncthreads();
     if (w < NP) {
         const uint32_t* hist = a.hist + ((uint64_t)sg * NP + w) * 256;
@@ -428,22 +485,8 @@ __global__ void __launch_bounds__(PLAN_BLOCK) sort_plan_kernel(const __grid_cons
     if (n <= CAP) {
         plan = {0u, 1u, act};  // one window of the local step
     } else if (na >= 3) {
-        // As many samples as show a mean of CAP rows in some 250 pairs.
-        uint32_t m = 256;
-        while (m < PLAN_SAMPLES && (uint64_t)m * m < n / 8 && 4 * m <= n) m *= 2;
-        const uint64_t step = n / m;
+        const uint64_t long_run = CAP / 2 + n / KeyTraits<K>::LOC_RUN;
         const double rows_per_pair = 2.0 * (double)n / ((double)m * (double)(m - 1));
-        K smp[PLAN_PER];  // one sample from each of m equal parts, at a mixed offset
-        int cnt_s = 0;
-#pragma unroll
-        for (int u = 0; u < PLAN_PER; ++u) {
-            const uint32_t i = (uint32_t)u * PLAN_BLOCK + t;
-            smp[u] = 0;
-            if (i < m) {
-                smp[u] = source_key<K>(a, d, i * step + (uint64_t)((i * 2654435761u) >> 8) % step);
-                cnt_s = u + 1;
-            }
-        }
         // The local step costs about one and a half passes.
         uint32_t sched = 0;
         for (int k = 1; k + 2 <= na; ++k) {
@@ -456,10 +499,12 @@ __global__ void __launch_bounds__(PLAN_BLOCK) sort_plan_kernel(const __grid_cons
                 mean = (double)block_sum((ull)c * c, red) / (double)n;
                 many = __syncthreads_or(c > CAP + n / 2048);
             } else {
-                const SampleRuns runs = sample_runs<K>(smp, cnt_s, 8 * top, 2 * m - 1, tab, cnt, fst, red);
+                const SampleRuns runs = sample_runs<K>(smp, cnt_s, 8 * top, 2 * m - 1, tab, cnt, fst, reinterpret_cast<uint32_t*>(red));
                 mean = rows_per_pair * (double)runs.pairs;
-                // (one CTA sweeps a hot value's run: 1/64 of the rows at most)
-                many = (runs.longest >= 6 && runs.longest * step > CAP + n / 2048) || runs.hottest * step > n / 64;
+                // (one CTA sweeps a hot value's run, 4 * CAP rows in some
+                // 25 us: up to that or 1/64 of the rows)
+                many = (runs.longest >= 6 && runs.longest * step > long_run) ||
+                       runs.hottest * step > max((uint64_t)CAP * 4, n / 64);
             }
             if (!many && mean <= KeyTraits<K>::LOC_FULL * CAP) {
                 plan = {sched, 1u, act};

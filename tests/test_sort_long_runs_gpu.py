@@ -82,3 +82,21 @@ def test_crowded_window(bolt, engine, n, values):
     for x in (v, v >> 40, (v >> 32).astype(np.int32)):
         got, _ = _sort(bolt, engine, x)
         assert np.array_equal(got, np.argsort(x, kind="stable"))
+
+
+@pytest.mark.parametrize("n", [1_000_003, 3_000_017])
+@pytest.mark.parametrize("length", [8_000, 16_000])
+def test_long_run_is_seen(bolt, engine, n, length):
+    """A run of many values longer than a window, against keys that get a pass for every digit: the sample must see
+    the run before its one block takes longer than the passes left out."""
+    rng = np.random.default_rng(n + length)
+    v = _full(rng, n)
+    every = v.copy()
+    v[rng.permutation(n)[:length]] = (0x1111111 << 32) + rng.integers(0, 1 << 32, length)
+    got, ms = _sort(bolt, engine, v, 9)
+    assert np.array_equal(got, np.argsort(v, kind="stable"))
+    every[::2] = (every[::2] & 0xFFFF) + (5 << 40)
+    got, every_ms = _sort(bolt, engine, every, 9)
+    assert np.array_equal(got, np.argsort(every, kind="stable"))
+    print(f"{n} rows, run of {length}: {ms * 1e3:.1f} us, every digit {every_ms * 1e3:.1f}")
+    assert ms <= every_ms
