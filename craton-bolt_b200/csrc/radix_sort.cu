@@ -63,8 +63,11 @@ constexpr int LOC_NW = LOC_BLOCK / 32;
 constexpr int LOC_BINS_LOG2 = 14;  // bins of the local step, counted in bytes
 constexpr int LOC_WORDS = (1 << LOC_BINS_LOG2) / 4;
 // Keys one bin may hold (a byte counts them): every key is compared with the
-// others of its bin, so chunks with longer ones take local_merge_sort.
+// others of its bin, so chunks with longer ones take local_crowded_sort.
 constexpr uint32_t LOC_BIN_MAX = 32;
+// Distinct keys up to which a crowded chunk is sorted by digits first: 256 keys
+// spread over 2^16 cells meet in one in 40 % of the chunks, 362 in 63 %.
+constexpr uint32_t LOC_FEW = 256;
 constexpr int LOC_SER_ROUNDS = 4;  // 32-key rounds per warp and tile of the serial path
 
 template <typename K> struct KeyTraits;
@@ -904,27 +907,115 @@ struct Packer {
     __device__ __forceinline__ uint32_t operator()(uint32_t k) const { return __byte_perm(k, 0u, lo); }
 };
 
+// One stable counting pass of the crowded-chunk sort over the row numbers
+// src -> dst (identity: src is 0, 1, 2, ...), by digit(row).
+template <int ITEMS, class Digit>
+__device__ __forceinline__ void local_pass(const uint16_t* src, uint16_t* dst, bool identity, uint32_t len, uint32_t* cnt,
+                                           uint32_t* wsum, Digit digit) {
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+    for (int i = t; i < LOC_NW * 256; i += LOC_BLOCK) cnt[i] = 0;
+    __syncthreads();
+    uint32_t rd[ITEMS];  // row | digit << 16
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const uint32_t p = (uint32_t)(w * ITEMS + r) * 32 + lane;
+        rd[r] = 0;
+        if (p < len) {
+            const uint32_t id = identity ? p : src[p], dg = digit(id);
+            rd[r] = id | (dg << 16);
+            atomicAdd(&cnt[w * 256 + dg], 1u);
+        }
+    }
+    __syncthreads();
+    uint32_t run = 0, x = 0;
+    if (t < 256) {
+        for (int ww = 0; ww < LOC_NW; ++ww) run += cnt[ww * 256 + t];
+        x = run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) wsum[w] = x;
+    }
+    __syncthreads();
+    if (t < 256) {
+        uint32_t off = x - run;
+        for (int i = 0; i < w; ++i) off += wsum[i];
+        for (int ww = 0; ww < LOC_NW; ++ww) {
+            const uint32_t c = cnt[ww * 256 + t];
+            cnt[ww * 256 + t] = off;
+            off += c;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const uint32_t p = (uint32_t)(w * ITEMS + r) * 32 + lane;
+        const bool in = p < len;
+        const uint32_t dg = rd[r] >> 16;
+        uint32_t peers = __ballot_sync(0xffffffffu, in);
+#pragma unroll
+        for (int bit = 0; bit < 8; ++bit) {
+            const uint32_t on = (dg >> bit) & 1u;
+            const uint32_t bal = __ballot_sync(0xffffffffu, on);
+            peers &= on ? bal : ~bal;
+        }
+        uint32_t b = 0;
+        if (in) b = cnt[w * 256 + dg];
+        __syncwarp();
+        if (in) {
+            if (lane == 31 - __clz(peers)) cnt[w * 256 + dg] = b + __popc(peers);
+            dst[b + __popc(peers & lanemask_lt())] = (uint16_t)(rd[r] & 0xFFFFu);
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+}
+
 // Sorts a chunk whose keys crowd into too few bins (repeated keys, or gaps
 // between clusters), in shared memory: skey holds its keys in chunk order,
-// spay the payloads; payloads from gap_at on go `gap` places further. A stable
-// merge sort of the row numbers (ia, ib): each thread sorts LOC_ITEMS
-// neighbours in registers, then pairs of lists are merged, each thread its own
-// LOC_ITEMS outputs of a pair from where a binary search says they begin. Its
-// cost is the same for all keys, and short, since the grid ends with its
-// slowest chunk (2M floats with 2,000 of each special value: local step 64 us
-// with two to ten counting passes here, 50 us; 32 us without such values).
+// spay the payloads; payloads from gap_at on go `gap` places further. Row
+// numbers (ia, ib) are sorted. A few keys that repeat (digits) are settled by
+// two stable counting passes over the leading 16 bits of the keys' range;
+// where those do not leave the rows in order, and for many keys straight away,
+// a stable merge sort does it: each thread sorts LOC_ITEMS neighbours in
+// registers, then pairs of lists are merged, each thread its own LOC_ITEMS
+// outputs of a pair from where a binary search says they begin; lists in order
+// are only copied, as most are once they are longer than the runs. (With two
+// CTAs per SM at it, the counting passes take 26 us a chunk, the merge sort
+// 40-50: 10M prices of 100,000 values 610 us, by merging alone 760. Where the
+// passes do not settle it, up to eight more took 53 us: 5M floats with 0.4 %
+// special values 313 us, by merging alone 278, every digit in a pass 280.)
 template <typename K>
-__device__ __noinline__ void local_merge_sort(const K* skey, const uint32_t* spay, uint16_t* ia, uint16_t* ib, uint32_t len,
-                                              uint32_t* out, uint32_t gap_at, uint64_t gap) {
+__device__ __noinline__ void local_crowded_sort(const K* skey, const uint32_t* spay, uint16_t* ia, uint16_t* ib, uint32_t len,
+                                                bool digits, uint32_t act, K lo, int bits, uint32_t* out, uint32_t gap_at,
+                                                uint64_t gap, uint32_t* cnt, uint32_t* wsum) {
     constexpr uint32_t ITEMS = KeyTraits<K>::LOC_ITEMS;
     const uint32_t t = threadIdx.x;
+    if (digits) {
+        const Packer pack(act, (int)sizeof(K));
+        const int top = bits > 16 ? bits - 16 : 0;
+        local_pass<ITEMS>(ia, ia, true, len, cnt, wsum, [&](uint32_t i) { return (uint32_t)((K)(pack(skey[i]) - lo) >> top) & 0xFFu; });
+        local_pass<ITEMS>(ia, ib, false, len, cnt, wsum,
+                          [&](uint32_t i) { return (uint32_t)((K)(pack(skey[i]) - lo) >> top >> 8) & 0xFFu; });
+        bool ok = true;
+        if (bits > 16)
+            for (uint32_t p = t + 1; p < len; p += LOC_BLOCK) ok = ok && skey[ib[p - 1]] <= skey[ib[p]];
+        if (__syncthreads_and(ok)) {
+            for (uint32_t p = t; p < len; p += LOC_BLOCK) out[p + (p >= gap_at ? gap : 0)] = spay[ib[p]];
+            __syncthreads();
+            return;
+        }
+    }
     {
         K k[ITEMS];
         uint32_t id[ITEMS];
 #pragma unroll
         for (uint32_t j = 0; j < ITEMS; ++j) {
-            id[j] = t * ITEMS + j;
-            k[j] = id[j] < len ? skey[id[j]] : ~(K)0;  // (rows past the end stay behind equal keys)
+            const bool in = t * ITEMS + j < len;
+            id[j] = !in ? 0u : digits ? ib[t * ITEMS + j] : t * ITEMS + j;
+            k[j] = in ? skey[id[j]] : ~(K)0;  // (rows past the end stay behind equal keys)
         }
 #pragma unroll
         for (uint32_t r = 0; r < ITEMS; ++r) {  // odd-even transposition: neighbours only, so it is stable
@@ -991,7 +1082,7 @@ __device__ __noinline__ void local_merge_sort(const K* skey, const uint32_t* spa
 // A run longer than a window (len rows at kin / pin) in which one value is
 // frequent: a sweep counts the rows below and equal to it, a second one writes
 // the equal rows' payloads in place and collects the others, in order, to be
-// sorted around the gap: at skey / spay by local_merge_sort where they fit a
+// sorted around the gap: at skey / spay by local_crowded_sort where they fit a
 // window, else in the run's part of the other buffer (kalt / palt) by
 // local_serial_sort, with the run's own part, read for the last time, for its
 // row numbers. So a run costs two sweeps and the sort of its other rows,
@@ -1070,7 +1161,7 @@ __device__ __forceinline__ bool local_hot_run(K* kin, uint32_t* pin, K* kalt, ui
     }
     __syncthreads();
     if (fits)
-        local_merge_sort<K>(skey, spay, ia, ia + cap, (uint32_t)n_rest, out, (uint32_t)below, equal);
+        local_crowded_sort<K>(skey, spay, ia, ia + cap, (uint32_t)n_rest, false, 0u, (K)0, 0, out, (uint32_t)below, equal, cnt, wsum);
     else
         local_serial_sort<K>(kalt, palt, reinterpret_cast<uint32_t*>(kin), pin, n_rest, out, below, equal, cnt, base, red);
     return true;
@@ -1127,7 +1218,7 @@ __global__ void __launch_bounds__(LOC_BLOCK, 2) sort_local_kernel(const __grid_c
     uint32_t* spay = bins + LOC_WORDS;                         // payloads in chunk order
     uint32_t* smeta = spay + CAP;                              // binned: position in the chunk, bin's length << 16, arrival << 24
     uint16_t* woff = reinterpret_cast<uint16_t*>(smeta + CAP);  // LOC_WORDS: keys before each word's bins
-    __shared__ uint32_t s_item, s_heavy, s_last;
+    __shared__ uint32_t s_item, s_heavy, s_used, s_last;
     __shared__ uint64_t s_lim[2];
     __shared__ uint32_t s_wsum[LOC_NW];
     __shared__ ull red[2 * LOC_NW];
@@ -1137,8 +1228,10 @@ __global__ void __launch_bounds__(LOC_BLOCK, 2) sort_local_kernel(const __grid_c
         __syncthreads();
         if (t == 0) s_item = atomicAdd(&a.tile_ctr[KeyTraits<K>::NPASS], 1u);
         __syncthreads();
-        const uint32_t item = s_item;
-        if (item >= a.total_loc_items) return;
+        if (s_item >= a.total_loc_items) return;
+        // Infinities and NaNs, the likeliest crowded chunks, go first: their
+        // longer sort is then not what the grid ends with.
+        const uint32_t item = a.desc ? s_item : a.total_loc_items - 1 - s_item;
         const int sg = seg_of(a.loc_begins, a.nseg, item);
         const SegDesc& d = seg_desc(a, sg);
         const SegPlan plan = a.plan[sg];
@@ -1251,7 +1344,7 @@ __global__ void __launch_bounds__(LOC_BLOCK, 2) sort_local_kernel(const __grid_c
             const int bits = sizeof(K) == 8 ? 64 - __clzll((ll)span) : 32 - __clz((int)span);
             const int bsh = bits > LOC_BINS_LOG2 ? bits - LOC_BINS_LOG2 : 0;
             for (int i = t; i < LOC_WORDS / 4; i += LOC_BLOCK) reinterpret_cast<uint4*>(bins)[i] = make_uint4(0, 0, 0, 0);
-            if (t == 0) s_heavy = 0;
+            if (t == 0) s_heavy = s_used = 0;
             __syncthreads();
             uint32_t br[ITEMS];  // bin | arrival number in the bin << 16
             bool heavy = false;
@@ -1269,14 +1362,26 @@ __global__ void __launch_bounds__(LOC_BLOCK, 2) sort_local_kernel(const __grid_c
             if (heavy) s_heavy = 1;
             __syncthreads();
             if (s_heavy) {
+                // Distinct keys: flags by hash, in woff's 8,192 bytes.
+                uint4* flags = reinterpret_cast<uint4*>(woff);
+                static_assert(LOC_WORDS * 2 == LOC_BLOCK * 16, "one uint4 of flags a thread");
+                flags[t] = make_uint4(0, 0, 0, 0);
+                __syncthreads();
 #pragma unroll
                 for (int j = 0; j < ITEMS; ++j) {
                     const uint32_t i = (uint32_t)j * LOC_BLOCK + t;
-                    if (i < len) skey[i] = key[j];
+                    if (i >= len) continue;
+                    skey[i] = key[j];
+                    reinterpret_cast<uint8_t*>(woff)[((ull)key[j] * 0x9E3779B97F4A7C15ull) >> 51] = 1;
                 }
                 __syncthreads();
+                const uint4 q = flags[t];
+                const uint32_t used = __reduce_add_sync(0xffffffffu, __popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w));
+                if (lane == 0) atomicAdd(&s_used, used);
+                __syncthreads();
                 uint16_t* ia = reinterpret_cast<uint16_t*>(smeta);
-                local_merge_sort<K>(skey, spay, ia, ia + CAP, len, d.payload_out + pos, len, 0);
+                local_crowded_sort<K>(skey, spay, ia, ia + CAP, len, s_used > 1 && s_used <= LOC_FEW, plan.act, lo, bits, d.payload_out + pos,
+                                      len, 0, bins, s_wsum);
                 pos += len;
                 continue;
             }
