@@ -23,3 +23,49 @@ def test_lengths_around_the_hand_over(bolt, engine, oracle, lengths):
     res = engine.execute_groupby(dev, ["k0", "k1"], AGGS)
     assert res.n_groups == len(lengths)
     _check(res, oracle.groupby_wide(host, ["k0", "k1"], AGGS), AGGS)
+
+
+def _lengths(n_groups, long_at):
+    """1 or 2 rows a group, but for the groups of long_at: {group: rows}."""
+    lengths = 1 + np.arange(n_groups) % 2
+    for g, rows in long_at.items():
+        lengths[g] = rows
+    return lengths
+
+
+def _by_length(bolt, oracle, rng, lengths):
+    group = rng.permutation(np.repeat(np.arange(len(lengths)), lengths))
+    cols = _columns(rng, len(group), ("i64", "i32"), 1, key_nulls=False)
+    cols["k0"] = ((group >> 4).astype(np.int64) * (1 << 35) - 5, None, "i64")
+    cols["k1"] = ((group & 15).astype(np.int32), None, "i32")
+    return _tables(bolt, oracle, cols)
+
+
+def test_long_groups_among_many(bolt, engine, oracle):
+    """More groups than 32 a warp of the grid (148 SMs x 64 warps): long ones next to each other, at the ends of the
+    grid's rounds (9,472 warps) and of 32 rounds (303,104 groups), and the very last."""
+    n_groups = 350_011
+    warps = 148 * 64
+    long_at = {g: 49 + 251 * i // 40 for i, g in enumerate(
+        [0, 1, 2, 31, 32, 33, 63, 64, warps - 1, warps, warps + 1, 2 * warps, 31 * warps - 1, 31 * warps, 32 * warps - 2,
+         32 * warps - 1, 32 * warps, 32 * warps + 1, 33 * warps] + list(range(200_000, 200_016)) + [n_groups - 2, n_groups - 1])}
+    rng = np.random.default_rng(2)
+    dev, host = _by_length(bolt, oracle, rng, _lengths(n_groups, long_at))
+    res = engine.execute_groupby(dev, ["k0", "k1"], AGGS)
+    assert res.n_groups == n_groups
+    _check(res, oracle.groupby_wide(host, ["k0", "k1"], AGGS), AGGS)
+
+
+def test_long_neighbours_fold_side_by_side(bolt, engine, oracle):
+    """Sixteen long groups next to each other in key order, among more groups than 32 a warp: their folds are chains
+    of dependent adds and must not follow one another, so together they take little more than one of them."""
+    n_groups, rows = 350_011, 60_000
+    ms = []
+    for long_at in ({200_000: rows}, {200_000 + i: rows for i in range(16)}):
+        dev, _ = _by_length(bolt, oracle, np.random.default_rng(3), _lengths(n_groups, long_at))
+        least = []
+        for _ in range(3):
+            assert engine.execute_groupby(dev, ["k0", "k1"], [("sum", "vd")], groups_hint=n_groups).n_groups == n_groups
+            least.append(engine.last_device_ms)
+        ms.append(min(least))
+    assert ms[1] <= 3 * ms[0]
