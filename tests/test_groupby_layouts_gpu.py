@@ -65,3 +65,19 @@ def test_layouts_share_a_batch(bolt, engine, oracle):
         assert r.n_groups == alone.n_groups
         for x, y in zip(r.keys + r.aggs, alone.keys + alone.aggs):
             assert np.array_equal(x.numpy(), y.numpy(), equal_nan=x.dtype == "f64")
+
+
+@pytest.mark.parametrize("n,count,own", [(3_000, 8, False), (900_000, 8, False), (1 << 20, 8, True), (400_000, 2, False),
+                                         (900_000, 2, True), (3_000, 1, True)])
+def test_batch_launches(bolt, engine, n, count, own):
+    """A batch of several layouts costs one aggregation launch where they have few rows, and one a layout where the
+    row loops compiled for them pay for it."""
+    cols = _columns(n, 50, n)
+    dev = {k: bolt.col(d, dt, v, s).to("cuda") for k, (d, v, dt, s) in cols.items()}
+
+    def launches(layouts):
+        engine.execute_batch([engine.prepare_groupby(dev, ["k"], a, groups_hint=101) for a in layouts])
+        return engine.last_launches
+
+    some = list(LAYOUTS.values())[:count]
+    assert launches(some) - launches([some[0]] * count) == (count - 1 if own else 0)
