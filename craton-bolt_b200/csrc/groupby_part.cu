@@ -912,6 +912,7 @@ bool gb_lean_applies(const GbPlan& pl, uint32_t flags) {
 bool gb_part_applies(const bolt_ctx* ctx, const GbPlan& pl, uint32_t flags) {
     (void)ctx;
     if ((flags & BOLT_FLAG_NO_PART) || !gb_lean_applies(pl, flags)) return false;
+    if (!reduce_kernel_for(pl.prm.spec)) return false;  // a layout that only the global-table tier compiles
     // Used when forced, or when the autotuner found it the faster tier for
     // this query shape (and the shape expects many groups).
     const bool forced = (flags & BOLT_FLAG_FORCE_PART) != 0;

@@ -4,8 +4,11 @@ kernel's start and off every tile."""
 
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 import pytest
+import torch
 
 from helpers import bitmap
 from test_groupby_gpu import run_both
@@ -81,3 +84,30 @@ def test_batch_launches(bolt, engine, n, count, own):
 
     some = list(LAYOUTS.values())[:count]
     assert launches(some) - launches([some[0]] * count) == (count - 1 if own else 0)
+
+
+@pytest.mark.parametrize("layout,tier", [("sum_i64", 1), ("avg3", 1), ("sum2_i64", 1), ("count_avg", 2)])
+def test_partitioned_tier_on_request(bolt, engine, layout, tier):
+    """The partitioned tier is asked for, but serves only the layouts it compiles; another one is planned for the
+    global table straight away: as many graph nodes when captured as without the request."""
+    from cuda.bindings import runtime as rt
+
+    n = 500_003
+    dev = {k: bolt.col(d, dt, v, s).to("cuda") for k, (d, v, dt, s) in _columns(n, 20_000, 3).items()}
+    aggs = {**LAYOUTS, "count_avg": [("count_star", None), ("avg", "x")]}[layout]
+    pq = engine.prepare_groupby(dev, ["k"], aggs, groups_hint=100_000)
+    engine.execute_batch([pq])
+
+    def nodes(flags):
+        graph, stream = torch.cuda.CUDAGraph(keep_graph=True), torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+            st = engine._lib.bolt_groupby(engine._ctx, C.byref(pq.desc), C.byref(pq.out), flags | bolt.FLAG_ASYNC,
+                                          C.c_void_p(stream.cuda_stream))
+        assert st == 0 and engine.last_groupby_tier == (tier if flags else 1)
+        err, _, count = rt.cudaGraphGetNodes(rt.cudaGraph_t(graph.raw_cuda_graph()))
+        assert err == rt.cudaError_t.cudaSuccess
+        return count
+
+    plain = [nodes(0), nodes(0)][1]  # (a kernel's first use can add one)
+    asked = [nodes(bolt.FLAG_FORCE_PART), nodes(bolt.FLAG_FORCE_PART)][1]
+    assert (asked == plain) == (tier == 1)
