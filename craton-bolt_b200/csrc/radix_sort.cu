@@ -145,7 +145,7 @@ struct SortArgs {
     uint32_t total_loc_items;
     uint32_t loc_range;    // rows of one work item of the local step
     uint32_t* tile_ctr;    // NPASS + 2 (the last two: the local step's items, long runs found)
-    LongRun* longs;
+    LongRun* longs;        // in the look-back words, which the last pass is done with
     uint32_t max_longs;
     uint32_t* status;
 };
@@ -1275,11 +1275,13 @@ __global__ void __launch_bounds__(LOC_BLOCK, 2) sort_local_kernel(const __grid_c
             }
             // The next window on its way to L2 meanwhile.
             if (t == 0 && end - pos > win) {
-                const uint64_t p0 = (pos + win) & ~7ull;
-                const uint32_t rows = (uint32_t)(end - p0 < CAP ? end - p0 : CAP) & ~7u;
-                if (rows) {
-                    bulk_prefetch_l2(kin + p0, rows * (uint32_t)sizeof(K));
-                    bulk_prefetch_l2(pin + p0, rows * 4u);
+                // (whole groups of 8 rows of the buffers, which start on
+                // 256-byte boundaries: 16-byte aligned addresses and sizes)
+                const uint64_t next = pos + win, stop = end - next < CAP ? end : next + CAP;
+                const uint64_t b0 = (d.buf_off + next) & ~7ull, b1 = (d.buf_off + stop) & ~7ull;
+                if (b0 < b1) {
+                    bulk_prefetch_l2((const K*)(in_a ? a.kA : a.kB) + b0, (uint32_t)(b1 - b0) * (uint32_t)sizeof(K));
+                    bulk_prefetch_l2((in_a ? a.pA : a.pB) + b0, (uint32_t)(b1 - b0) * 4u);
                 }
             }
             // The chunk: the window up to its last run start, or all of it
@@ -1466,7 +1468,7 @@ bolt_status run_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
     if (nseg == 0) return BOLT_OK;
     std::vector<SegDesc> segs(nseg);
     std::vector<uint32_t> begins(3 * (nseg + 1));
-    uint64_t total_n = 0, end_n = 0, items = 0, hitems = 0, litems = 0;
+    uint64_t total_n = 0, items = 0, hitems = 0, litems = 0;
     // Rows of one local work item: a few chunks, so that finding its ends is
     // a small part of it, but enough items for every CTA.
     uint64_t sum_n = 0;
@@ -1482,8 +1484,7 @@ bolt_status run_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
         begins[i] = (uint32_t)items;
         begins[nseg + 1 + i] = (uint32_t)hitems;
         begins[2 * (nseg + 1) + i] = (uint32_t)litems;
-        end_n = total_n + g.n;
-        total_n += (g.n + 15) & ~15ull;  // (16-byte aligned buffers for the local step's prefetches)
+        total_n += g.n;
         items += (g.n + SORT_TILE - 1) / SORT_TILE;
         hitems += (g.n + HIST_CHUNK - 1) / HIST_CHUNK;
         litems += (g.n + loc_range - 1) / loc_range;
@@ -1504,7 +1505,7 @@ bolt_status run_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
     a.total_loc_items = (uint32_t)litems;
     a.loc_range = (uint32_t)loc_range;
     a.lb_stride = items * 256;
-    const uint64_t nb = end_n ? end_n : 1;
+    const uint64_t nb = total_n ? total_n : 1;
     const bool many = nseg > 1;
     SegDesc* d_segs = many ? (SegDesc*)arena_alloc(ctx, sizeof(SegDesc) * nseg) : nullptr;
     uint32_t* d_begins = many ? (uint32_t*)arena_alloc(ctx, 4 * begins.size()) : nullptr;
@@ -1519,9 +1520,10 @@ bolt_status run_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
     a.tile_ctr = (uint32_t*)arena_alloc(ctx, 64);
     constexpr uint64_t LOC_CAP = (uint64_t)LOC_BLOCK * KeyTraits<K>::LOC_ITEMS;
     a.max_longs = (uint32_t)(sum_n / LOC_CAP + 1);
-    a.longs = (LongRun*)arena_alloc(ctx, a.max_longs * sizeof(LongRun));
+    a.longs = reinterpret_cast<LongRun*>(a.lookback);
+    static_assert(sizeof(LongRun) * 2 <= 256 * 4 && LOC_CAP >= (uint64_t)SORT_TILE, "the look-back words of a sort hold its long runs");
     a.status = ctx->d_status;
-    if (!a.longs || (many && (!d_segs || !d_begins)) || !a.kA || !a.kB || !a.pA || !a.pB || !a.hist || !a.digit_base || !a.plan ||
+    if ((many && (!d_segs || !d_begins)) || !a.kA || !a.kB || !a.pA || !a.pB || !a.hist || !a.digit_base || !a.plan ||
         !a.lookback || !a.tile_ctr)
         return fail(ctx, BOLT_ERR_CAPACITY, "radix sort: scratch arena too small for %llu rows", (ull)total_n);
     a.segs = d_segs;
@@ -1567,7 +1569,7 @@ bolt_status run_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
 uint64_t radix_sort_scratch(uint64_t total_n, uint64_t nseg, int32_t src) {
     const uint64_t ksz = (src == SRC_I32 || src == SRC_F32 || src == SRC_U32) ? 4 : 8;
     const uint64_t items = total_n / SORT_TILE_MIN + nseg + 1;
-    return 2 * total_n * (ksz + 4) + total_n / 200 + 2 * items * 256 * 4 + nseg * (2 * 8 * 256 * 4 + 512) + 64 * 1024;
+    return 2 * total_n * (ksz + 4) + 2 * items * 256 * 4 + nseg * (2 * 8 * 256 * 4 + 96) + 64 * 1024;
 }
 
 bolt_status radix_sort(bolt_ctx* ctx, cudaStream_t s, const SortSpec& sp) {
