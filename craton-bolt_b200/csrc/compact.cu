@@ -619,7 +619,9 @@ __global__ void __launch_bounds__(1024) compact_scan_kernel(const __grid_constan
 // gathered once: this pass packs them in element order and counts each
 // 2,048-row tile's, and split_write_kernel places both parts from the packed
 // bits. (Two compactions, each gathering in both of its passes: 257 us for
-// 10M rows.)
+// for 10M rows.) Without room for the packed bits (PACKED false) the second
+// pass gathers them again.
+template <bool PACKED>
 __global__ void __launch_bounds__(CP_BLOCK) split_count_kernel(const __grid_constant__ CpArgs a, const uint32_t* ids_in,
                                                                uint32_t* bits) {
     constexpr int TILE = CP_BLOCK * CP_ITEMS_DIRECT;
@@ -638,7 +640,7 @@ __global__ void __launch_bounds__(CP_BLOCK) split_count_kernel(const __grid_cons
     for (int j = 0; j < CP_ITEMS_DIRECT; ++j) {
         const uint64_t e = base + (uint64_t)j * CP_BLOCK + threadIdx.x;
         const uint32_t m = __ballot_sync(0xffffffffu, e < sp.n && bit_valid(sp.keep_valid_of, id[j]));
-        if (lane == 0) bits[e >> 5] = m;  // (whole tiles of words are allocated)
+        if (PACKED && lane == 0) bits[e >> 5] = m;  // (whole tiles of words are allocated)
         c += __popc(m);
     }
     if (lane == 0) wcnt[w] = c;
@@ -653,6 +655,7 @@ __global__ void __launch_bounds__(CP_BLOCK) split_count_kernel(const __grid_cons
 
 // sp.row_ids receives the valid ids; `nulls` the others, from row 0
 // (nulls_first) or from the number of valid rows.
+template <bool PACKED>
 __global__ void __launch_bounds__(CP_BLOCK) split_write_kernel(const __grid_constant__ CpArgs a, const uint32_t* ids_in,
                                                                const uint32_t* bits, uint32_t* nulls, int nulls_first, uint32_t ntiles) {
     constexpr int TILE = CP_BLOCK * CP_ITEMS_DIRECT, WORDS = TILE / 32;
@@ -662,13 +665,23 @@ __global__ void __launch_bounds__(CP_BLOCK) split_write_kernel(const __grid_cons
     const int lane = threadIdx.x & 31;
     const uint32_t tile = blockIdx.x;
     const uint64_t base = (uint64_t)tile * TILE;
+    if (!PACKED) {
+#pragma unroll
+        for (int j = 0; j < CP_ITEMS_DIRECT; ++j) {
+            const uint32_t i = (uint32_t)j * CP_BLOCK + threadIdx.x;
+            const uint64_t e = base + i;
+            const uint32_t m = __ballot_sync(0xffffffffu, e < sp.n && bit_valid(sp.keep_valid_of, ids_in ? __ldg(ids_in + e) : e));
+            if (lane == 0) word[i >> 5] = m;
+        }
+        __syncthreads();
+    }
     if (threadIdx.x < 32) {
         ull total;
         const ull b = cp_two_base(a, tile, ntiles, &total);
         uint32_t run = 0;
 #pragma unroll
         for (int h = 0; h < WORDS; h += 32) {
-            const uint32_t m = bits[base / 32 + h + lane], c = __popc(m);
+            const uint32_t m = PACKED ? bits[base / 32 + h + lane] : word[h + lane], c = __popc(m);
             uint32_t x = c;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -826,11 +839,15 @@ bolt_status null_split_enqueue(bolt_ctx* ctx, cudaStream_t s, uint64_t n, const 
     const uint64_t mark = ctx->arena_used;  // (scratch of these launches only: later work on the stream may reuse it)
     a.group_tot = (ull*)arena_alloc(ctx, (groups + 1) * 8 + ntiles * 4);
     a.tile_cnt = reinterpret_cast<uint32_t*>(a.group_tot + ((groups + 1) & ~1ull));
+    if (!a.group_tot) return fail(ctx, BOLT_ERR_CAPACITY, "NULL split: scratch arena too small");
+    // (A column of hardly more than NULLs sorts in little more than its valid
+    // ids: the bits may be what does not fit.)
     uint32_t* bits = (uint32_t*)arena_alloc(ctx, ntiles * TILE / 8);
-    if (!a.group_tot || !bits) return fail(ctx, BOLT_ERR_CAPACITY, "NULL split: scratch arena too small");
-    split_count_kernel<<<(unsigned)ntiles, CP_BLOCK, 0, s>>>(a, ids_in, bits);
+    if (bits) split_count_kernel<true><<<(unsigned)ntiles, CP_BLOCK, 0, s>>>(a, ids_in, bits);
+    else split_count_kernel<false><<<(unsigned)ntiles, CP_BLOCK, 0, s>>>(a, ids_in, bits);
     compact_scan_kernel<<<(unsigned)groups, 1024, 0, s>>>(a, (uint32_t)ntiles);
-    split_write_kernel<<<(unsigned)ntiles, CP_BLOCK, 0, s>>>(a, ids_in, bits, nulls, nulls_first ? 1 : 0, (uint32_t)ntiles);
+    auto write = bits ? split_write_kernel<true> : split_write_kernel<false>;
+    write<<<(unsigned)ntiles, CP_BLOCK, 0, s>>>(a, ids_in, bits, nulls, nulls_first ? 1 : 0, (uint32_t)ntiles);
     ctx->arena_used = mark;
     ctx->last_launches += 3;
     BOLT_CUDA(ctx, cudaGetLastError());
