@@ -67,7 +67,7 @@ def test_crowded_window_costs_little(bolt, engine):
     got, ms = _sort(bolt, engine, v, 25)
     assert np.array_equal(got, np.argsort(v, kind="stable"))
     print(f"crowded {ms * 1e3:.1f} us, uniform {uniform_ms * 1e3:.1f}")
-    assert ms <= 1.5 * uniform_ms
+    assert ms - uniform_ms <= 0.032  # (38 us with a counting pass per digit, 26 by merging)
 
 
 # 5,120 rows: one window; 10 rows: what one thread sorts by itself.
