@@ -579,6 +579,34 @@ def join_probe_host(dg, npr: int, nb: int) -> dict:
 # ---------------------------------------------------------------------------
 # Workloads: ORDER BY radix sort
 # ---------------------------------------------------------------------------
+def sort_schedule(keys: np.ndarray, n: int):
+    """(digit passes, whether a local step follows) of n keys distributed like `keys`, by the library's rule: one
+    window of the local step by itself; the top digits whose runs of equal digits it holds; else every varying digit."""
+    kb = keys.dtype.itemsize
+    window, full = (5120, 0.9) if kb == 8 else (6144, 0.8)
+    if n <= window:
+        return 0, True
+    m = min(len(keys), 1 << 22)
+    raw = np.ascontiguousarray(keys[np.linspace(0, len(keys) - 1, m).astype(np.int64)])
+    u = raw.view(f"u{kb}").copy()
+    sign = u.dtype.type(1 << (8 * kb - 1))
+    u = np.where(u & sign, ~u, u | sign) if keys.dtype.kind == "f" else u ^ sign
+    varying = [p for p in range(kb) if ((u ^ u[0]) >> u.dtype.type(8 * p) & u.dtype.type(255)).any()]
+    for k in range(1, len(varying) - 1):
+        runs = np.unique(u >> u.dtype.type(8 * varying[-k]), return_counts=True)[1].astype(np.float64)
+        if n * (runs * (runs - 1)).sum() / (m * (m - 1.0)) <= full * window:
+            return k, True
+    return max(1, len(varying)), False
+
+
+def sort_bytes(n: int, kb: int, passes: int, local: bool) -> int:
+    """Bytes of one sort: the histogram reads the keys; a pass reads and writes key and u32 payload, but the first
+    generates its payload; the local step reads both and writes the payload, as the last pass does without one."""
+    moved = kb + (passes * 2 * (kb + 4) - 4 if passes else 0)
+    moved += (kb + 4 + 4 if passes else kb + 4) if local else -kb
+    return n * moved
+
+
 def w_sort(c: Ctx, kind: str):
     a = c.args
     torch = c.torch
@@ -607,13 +635,10 @@ def w_sort(c: Ctx, kind: str):
         return int(c.lib.bolt_ctx_last_launches(c.eng._ctx))
 
     ms, launches, kms, clocks = c.timed(step, a.steps, a.warmup)
-    # pass accounting for the short schedule these spread-out keys get: the
-    # histogram reads keys once; two 8-bit passes read and write (key + u32
-    # payload), the first reading only the key; the local step reads both and
-    # writes the payload.
-    passes = 2
-    alg = n * (kb + (kb + kb + 4) + 2 * (kb + 4) + (kb + 4 + 4))
-    line = base_line(c, ms, n, alg, kms, "sort (histogram, two digit passes, local step)", f"sort_{kind}",
+    passes, local = sort_schedule(keys, n)
+    alg = sort_bytes(n, kb, passes, local)
+    line = base_line(c, ms, n, alg, kms, f"sort (histogram, {passes} digit passes{', local step' if local else ''})",
+                     f"sort_{kind}",
                      {"workload": f"ORDER BY radix sort: {n} {dt} keys" +
                                   (" uniform over the full range" if kind == "i64" else
                                    " incl. negatives, +-0, +-inf, 0.1% NaN"),

@@ -85,3 +85,23 @@ def test_reference_arm_other_ranks_exit_quietly():
     r = _reference_arm(1)
     assert r.returncode == 0, r.stderr
     assert r.stdout.strip() == ""
+
+
+def test_sort_schedule_and_bytes():
+    """The byte count of the sort lines follows the passes that the library schedules for the size at hand."""
+    import numpy as np
+
+    sys.path.insert(0, str(REPO))
+    import bench
+
+    rng = np.random.default_rng(0)
+    full = rng.integers(-(1 << 63), (1 << 63) - 1, 1 << 20, dtype=np.int64)
+    assert [bench.sort_schedule(full, n) for n in (5000, 1_000_000, 1 << 25, 1 << 28, 400_000_000)] == \
+        [(0, True), (1, True), (2, True), (2, True), (3, True)]
+    assert bench.sort_schedule(full % 60_000, 1 << 25) == (2, False)
+    assert bench.sort_schedule(rng.normal(0, 1, 1 << 20).astype(np.float32), 1 << 30) == (4, False)
+    assert bench.sort_bytes(1, 8, 2, True) == 8 + 20 + 24 + 16
+    assert bench.sort_bytes(1, 8, 1, True) == 8 + 20 + 16
+    assert bench.sort_bytes(1, 8, 0, True) == 8 + 8 + 4
+    assert bench.sort_bytes(1, 8, 8, False) == 8 + 20 + 6 * 24 + 16
+    assert bench.sort_bytes(1, 4, 4, False) == 4 + 12 + 2 * 16 + 12
