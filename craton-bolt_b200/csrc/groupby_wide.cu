@@ -55,6 +55,7 @@ struct WideArgs {
     uint64_t n_groups;
     uint64_t n_kept;
     uint64_t n_write;         // groups written: min(n_groups, output capacity)
+    uint64_t thread_rows;  // (wide_thread_rows)
     int32_t n_aggs;
     WideAgg agg[GB_MAX_AGGS];
 };
@@ -128,11 +129,20 @@ __device__ __forceinline__ WideElem wide_elem(const WideArgs& a, const WideAgg& 
     return e;
 }
 
-// Groups up to this many rows are folded by one thread each, longer ones by
+// Groups up to thread_rows rows are folded by one thread each, longer ones by
 // one warp: a warp per group of ten rows leaves two thirds of its lanes idle
 // and walks its 32 shuffles for ten values (10M rows in 1M groups: 1,290 us, a
-// thread each 263 us).
+// thread each 263 us). A thread waits for its rows WIDE_TU at a time, though,
+// and gains only where the groups are several to a warp of the chip (64 warps
+// an SM): 12 aggregates of 48 rows a group, whole calls by threads and by
+// warps: 1,000 groups 503 and 385 us, 10,000 554 and 515, 40,000 713 and
+// 1,047; of 24 rows 398 and 370, 434 and 450, 489 and 723; of 12 rows 348 and
+// 335, 381 and 440, 406 and 681.
 constexpr uint64_t WIDE_THREAD_ROWS = 48;
+inline uint64_t wide_thread_rows(uint64_t n_groups, int num_sms) {
+    const uint64_t per_warp = (n_groups + (uint64_t)num_sms * 64 - 1) / ((uint64_t)num_sms * 64);
+    return std::min<uint64_t>(WIDE_THREAD_ROWS, 16 * per_warp - 8);
+}
 constexpr int WIDE_TU = 4;  // rows of a group in flight per thread
 
 // Writes aggregate q of group g (cnt valid inputs; the integer or the float
@@ -159,14 +169,14 @@ __device__ __forceinline__ void wide_store(const WideAgg& w, uint64_t g, uint64_
     if (w.out_valid) set_bit_atomic(w.out_valid, g, valid);
 }
 
-// One thread per group of at most WIDE_THREAD_ROWS rows: every aggregate in
+// One thread per group of at most thread_rows rows: every aggregate in
 // row order, WIDE_TU rows loaded before the first is folded.
 __global__ void __launch_bounds__(256) wide_fold_short_kernel(const __grid_constant__ WideArgs a) {
     const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < a.n_write; g += step) {
         const uint64_t beg = a.starts[g];
         const uint64_t end = g + 1 < a.n_groups ? a.starts[g + 1] : a.n_kept;
-        if (end - beg > WIDE_THREAD_ROWS) continue;
+        if (end - beg > a.thread_rows) continue;
         const uint32_t r0 = a.perm[beg];
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
@@ -246,7 +256,7 @@ __global__ void __launch_bounds__(256) wide_fold_kernel(const __grid_constant__ 
         bool is_long = false;
         if (gl < a.n_write) {
             const uint64_t e = gl + 1 < a.n_groups ? a.starts[gl + 1] : a.n_kept;
-            is_long = e - a.starts[gl] > WIDE_THREAD_ROWS;
+            is_long = e - a.starts[gl] > a.thread_rows;
         }
         uint32_t todo = __ballot_sync(0xffffffffu, is_long);
         while (todo) {
@@ -500,9 +510,10 @@ bolt_status gb_wide(bolt_ctx* ctx, const bolt_groupby_desc* d, bolt_groupby_out*
     wa.n_kept = n_kept;
     wa.n_write = std::min<uint64_t>(n_groups, out_cap);
     if (wa.n_write) {
+        wa.thread_rows = wide_thread_rows(wa.n_write, ctx->num_sms);
         wide_fold_short_kernel<<<grid_for(wa.n_write, 256, ctx->num_sms * 8), 256, 0, s>>>(wa);
         // (else no group is longer)
-        if (n_kept > WIDE_THREAD_ROWS) {
+        if (n_kept > wa.thread_rows) {
             const unsigned blocks = (unsigned)std::min<uint64_t>((wa.n_write + 7) / 8, (uint64_t)ctx->num_sms * 8);
             wide_fold_kernel<<<blocks, 256, 0, s>>>(wa);
             launches += 1;

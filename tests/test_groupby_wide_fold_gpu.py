@@ -69,3 +69,30 @@ def test_long_neighbours_fold_side_by_side(bolt, engine, oracle):
             least.append(engine.last_device_ms)
         ms.append(min(least))
     assert ms[1] <= 3 * ms[0]
+
+
+@pytest.mark.parametrize("n_groups", [9_471, 9_472, 9_473, 18_944, 18_945, 28_417])
+def test_hand_over_by_group_count(bolt, engine, oracle, n_groups):
+    """The length from which a warp folds a group rises with the groups per warp of the chip (148 x 64): 8, 24, 40,
+    48 rows. Groups of every length around them, in one query."""
+    edges = np.array([1, 2, 7, 8, 9, 23, 24, 25, 39, 40, 41, 47, 48, 49, 60])
+    lengths = np.where(np.arange(n_groups) % 19 == 0, edges[np.arange(n_groups) // 19 % len(edges)], 2)
+    rng = np.random.default_rng(n_groups)
+    dev, host = _by_length(bolt, oracle, rng, lengths)
+    res = engine.execute_groupby(dev, ["k0", "k1"], AGGS)
+    assert res.n_groups == n_groups
+    _check(res, oracle.groupby_wide(host, ["k0", "k1"], AGGS), AGGS)
+
+
+def test_few_short_groups_cost_no_more_than_longer_ones(bolt, engine, oracle):
+    """A thousand groups, every aggregate: 48 rows each against 49, which warps fold."""
+    ms = []
+    for rows in (48, 49):
+        dev, _ = _by_length(bolt, oracle, np.random.default_rng(4), np.full(1000, rows))
+        least = []
+        for _ in range(9):
+            engine.execute_groupby(dev, ["k0", "k1"], AGGS, groups_hint=1000)
+            least.append(engine.last_device_ms)
+        ms.append(min(least))
+    print(f"48 rows {ms[0] * 1e3:.1f} us, 49 rows {ms[1] * 1e3:.1f}")
+    assert ms[0] <= 1.1 * ms[1]
