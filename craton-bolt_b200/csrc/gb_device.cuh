@@ -334,7 +334,12 @@ __device__ __forceinline__ int s_find_insert(ull* sk, int log2, ull stored, uint
 // state kinds inside the unrolled row loop costs ~1,500 instructions per row
 // and thrashes the instruction cache; the common layouts (states sorted by
 // kind, see gb_plan) get a loop with the kinds known at compile time, and
-// everything else runs the generic loop.
+// everything else runs the generic loop. A layout is worth a loop of its own
+// (some 80 KB over the kernels) where plain queries ask for it: one to three
+// SUM / AVG of one type, with or without COUNT(*), one of them with NULLs, and
+// the benchmark's list with MIN and MAX. Mixed types, MIN or MAX without
+// COUNT(*) and longer lists run the generic loop, which takes two to three
+// times as long (10M rows, three AVGs: 794 us against 284).
 // ---------------------------------------------------------------------------
 struct SpecGeneric {
     static constexpr bool generic = true;

@@ -1628,7 +1628,7 @@ static bolt_status gb_run_tables(bolt_ctx* ctx, GbPlan** pls, int nq, cudaStream
 
 // Launches the aggregation of one query (the single-query kernels).
 static bolt_status gb_agg_one(bolt_ctx* ctx, GbPlan* pl, cudaStream_t s, uint32_t flags) {
-    // Dense shapes of 4M+ rows: the streaming kernel compiled for the key,
+    // Dense shapes of 256K+ rows: the streaming kernel compiled for the key,
     // WHERE and state layouts (groupby_part.cu), misses to the global table.
     if (!(flags & BOLT_FLAG_KERNEL_STAGED) && pl->tune.staged != 0) {
         bolt_status st = BOLT_OK;

@@ -53,7 +53,7 @@ struct alignas(16) GbPart {
 };
 
 // Whether the streaming kernel (compiled key / predicate / state layouts over
-// dense, 16-byte aligned columns of 4M+ rows) serves this planned query.
+// dense, 16-byte aligned columns of 256K+ rows) serves this planned query.
 bool gb_lean_applies(const GbPlan& pl, uint32_t flags);
 
 // Whether the partitioned tier serves this planned query.

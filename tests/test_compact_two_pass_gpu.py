@@ -1,5 +1,5 @@
-"""GPU parity of the two-pass row-id compaction (NULL split, run starts, unaligned columns) around the size it
-starts at and at the edges of its tiles, tile groups and scan rounds, against numpy, exactly."""
+"""GPU parity of the NULL split and of the two-pass row-id compaction (run starts, unaligned columns), around the
+size the two-pass form starts at and at the edges of their tiles and scan groups, against numpy, exactly."""
 
 from __future__ import annotations
 
@@ -11,8 +11,8 @@ from helpers import bitmap
 
 pytestmark = pytest.mark.gpu
 
-ROWS = 1 << 20  # the two-pass form starts here; 2,048-row tiles, 4 tiles a group, 16,384 counts a scan round
-SIZES = [ROWS - 1, ROWS, ROWS + 1, ROWS + 2048 * 3 + 7, 2048 * 16_384 + 2049]
+ROWS = 1 << 20  # the two-pass form starts here; 2,048-row tiles, 4,096 tiles a scan group
+SIZES = [ROWS - 1, ROWS, ROWS + 1, ROWS + 2048 * 3 + 7, 2048 * 4096 - 1, 2048 * 4096, 2048 * 4096 + 1, 2048 * 16_384 + 2049]
 
 
 @pytest.mark.parametrize("nulls_first", [False, True])

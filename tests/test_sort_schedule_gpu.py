@@ -40,7 +40,7 @@ def _keys(name: str, n: int) -> np.ndarray:
 NAMES = ["full", "narrow", "packed", "long_run", "one_value", "dups", "few", "sorted"]
 
 
-# 5,120 rows: one window of the local step; 8,192 samples; 32,768 rows: its largest work item.
+# 5,120 rows: one window of the local step; 4,096 rows: its work item at these sizes, ten of them and a row.
 @pytest.mark.parametrize("n", [33, 5119, 5120, 5121, 8191, 8193, 40_961, M])
 @pytest.mark.parametrize("name", NAMES)
 def test_i64(bolt, engine, name, n):
