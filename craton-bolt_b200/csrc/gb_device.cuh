@@ -282,10 +282,19 @@ __device__ __forceinline__ bool d128_value(const ull* w, __int128& v) {
 }
 
 // Global table find-or-insert; -1 (and SPILL) when the probe limit is hit.
+// LOOK: on a long chain it also gives up when the table is known to be too
+// small, since the attempt is then made again with a larger one. For the join
+// kernel: 25,000 probe rows of 4,597 groups met a full 4,096-slot table and
+// probed it for 4.1 ms of a 4.6 ms call (0.48 ms with LOOK). The loop costs
+// the streaming kernel 1 % (100M filtered rows 3,116 -> 3,154 us), unrolled in
+// any form 10-20 %.
+template <bool LOOK = false>
 __device__ __forceinline__ int64_t g_find_insert(const GbParams& p, ull stored, uint32_t& inserts) {
     const ull mask = (1ull << p.log2cap) - 1;
     ull h = (stored * HASH_G) >> (64 - p.log2cap);
     for (uint32_t i = 0; i < p.max_probe; ++i) {
+        if constexpr (LOOK)
+            if ((i & 31u) == 31u && (*reinterpret_cast<volatile uint32_t*>(p.status) & (ST_FLAG_GROW | ST_FLAG_SPILL))) return -1;
         ull* kp = p.gtab + h * (ull)p.slot_words;
         ull k = ld_volatile(kp);
         if (k == stored) return (int64_t)h;
@@ -417,13 +426,14 @@ __device__ __forceinline__ void gb_warp_flush_pending(const GbParams& p, uint32_
 
 // Merges a CTA's shared table into the query's global table (whole CTA,
 // after a __syncthreads()).
+template <bool LOOK = false>
 __device__ __forceinline__ void gb_flush_shared(const GbParams& p, const ull* sk, const ull* sw, int C) {
     const int SW = p.sslot_words - 1;
     uint32_t inserts = 0;
     for (int i = threadIdx.x; i < C; i += blockDim.x) {
         const ull key = sk[i];
         if (key == 0) continue;
-        const int64_t g = g_find_insert(p, key, inserts);
+        const int64_t g = g_find_insert<LOOK>(p, key, inserts);
         if (g < 0) continue;
         ull* w = p.gtab + (ull)g * p.slot_words;
         const ull* src = sw + (ull)i * SW - 1;

@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(512, 2) gb_join_lean_kernel(const __grid_const
             merge_words_smem(w + w0, K_COUNT, 1, 0, true);
             merge_words_smem(w + w1, KIND, c0, c1, true);
         } else {
-            const int64_t gs = g_find_insert(p, stored, inserts);
+            const int64_t gs = g_find_insert<true>(p, stored, inserts);
             if (gs < 0) {
                 look = true;
                 return;
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(512, 2) gb_join_lean_kernel(const __grid_const
     gb_warp_flush_pending(p, pending);
     gb_flush_absbits(p, absbits);
     __syncthreads();
-    gb_flush_shared(p, sk, sw, C);
+    gb_flush_shared<true>(p, sk, sw, C);
 }
 
 // ---------------------------------------------------------------------------
